@@ -128,4 +128,34 @@ DENSE_HD inline T div_by_count(T x, T c, T rc) {
   return x / c;
 }
 
+// x / c for a count c of at most kSmallCount, with rc = RN(1/c): the same
+// quotient without the proof, valid where small_count_operand(x).  For these
+// counts RN(1/c) is within 2^-p / 4 of 1/c relatively (p = 53 or 24; 1, 2
+// and 4 are exact, 3 and 6 are off by a third of an ulp of a mantissa of
+// 4/3, 5 by at most two fifths of an ulp of 8/5), so q0 = RN(x rc) is less
+// than one ulp from x/c, i.e. a faithful rounding, and then Markstein's
+// theorem (the paper cited above; also Muller et al., Handbook of
+// Floating-Point Arithmetic, ch. 4) makes q1 the correctly rounded quotient.
+constexpr int kSmallCount = 6;
+
+template <typename T>
+DENSE_HD inline T div_by_small_count(T x, T c, T rc) {
+  const T q0 = x * rc;
+  const T r0 = cd_fma(-q0, c, x);
+  return cd_fma(r0, rc, q0);
+}
+
+// Whether x is zero or of an exponent within [kLo, kHi) (integer tests on
+// the bits: cheaper on the device than floating comparisons).
+template <typename T>
+DENSE_HD inline bool small_count_operand(T x) {
+  using Tr = CountDivTraits<T>;
+  using Bits = typename Tr::Bits;
+  const Bits mag = Tr::bits(x) & ~(Bits(1) << (sizeof(T) * 8 - 1));
+  const uint32_t hi = static_cast<uint32_t>(mag >> (sizeof(T) * 8 - 32));
+  const uint32_t lo = static_cast<uint32_t>(Tr::bits(Tr::kLo) >> (sizeof(T) * 8 - 32));
+  const uint32_t top = static_cast<uint32_t>(Tr::bits(Tr::kHi) >> (sizeof(T) * 8 - 32));
+  return hi - lo < top - lo || mag == 0;
+}
+
 }  // namespace dense_b200

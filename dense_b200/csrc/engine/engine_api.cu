@@ -318,18 +318,27 @@ int plan_set(const dense_set_desc& in, double dt, int elem_bytes, SetPlan& plan,
   int widest = 0;
   for (size_t l = 0; l + 1 < plan.lvl_off.size(); ++l) widest = std::max(widest, plan.lvl_off[l + 1] - plan.lvl_off[l]);
   plan.mem_block = in.mem_block > 0 ? in.mem_block : std::min(256, std::max(32, (widest + 31) / 32 * 32));
+  // a power of two, so a row is (step - lag) & (D - 1); the wave kernel
+  // indexes rows modulo D and keeps exactly the rows it reads
   int64_t off = 0;
-  for (int sp = 0; sp < NUM_SPECIES; ++sp) {
-    int depth = 0;
-    if (own_max[sp] >= 1) depth = own_max[sp] + 1;
-    if (nbr_max[sp] >= 0) depth = std::max(depth, nbr_max[sp] + 2);
-    if (plan.use_mem) depth = std::max(depth, 2);
-    // a power of two, so a row is (step - lag) & (D - 1); the wave kernel
-    // indexes rows modulo D and keeps exactly the rows it reads
-    d.D[sp] = depth > 0 ? (plan.wave ? depth : next_pow2(depth)) : 0;
-    depth = d.D[sp];
-    d.ring_off[sp] = off;
-    off += static_cast<int64_t>(depth) * n;
+  auto stage = [&] {
+    off = 0;
+    for (int sp = 0; sp < NUM_SPECIES; ++sp) {
+      int depth = 0;
+      if (own_max[sp] >= 1) depth = own_max[sp] + 1;
+      if (nbr_max[sp] >= 0) depth = std::max(depth, nbr_max[sp] + 2);
+      if (plan.use_mem) depth = std::max(depth, 2);
+      d.D[sp] = depth > 0 ? (plan.wave ? depth : next_pow2(depth)) : 0;
+      d.ring_off[sp] = off;
+      off += static_cast<int64_t>(d.D[sp]) * n;
+    }
+  };
+  stage();
+  // the register kernel forms ring offsets in 32 bits and packs lags in 26;
+  // larger rings (no model's delays come near) go to the memory kernel
+  if (!plan.use_mem && off > kMaxRegisterRing) {
+    plan.use_mem = true;
+    stage();
   }
   // wave kernel shared memory, filled in priority order while it fits:
   // the rows of the species read at lag S-1, the FP32 Kahan terms (every
@@ -711,8 +720,8 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
   a.uniform_params = 1;
   for (const SetDesc& d : e->sets)
     if (d.param_stride != 0) a.uniform_params = 0;
-  // shared memory: sampled state (with analyses), truncated delays, and
-  // each set's neighbour ids when the largest list fits
+  // shared memory: sampled state (with analyses) and each set's neighbour
+  // ids when the largest list fits
   // rows of the sampled-state buffer: the species some analysis observes
   a.n_vals = 0;
   for (int sp = 0; sp < NUM_SPECIES; ++sp) a.val_slot[sp] = -1;
@@ -722,8 +731,7 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
   for (int i = 0; i < a.n_analyses; ++i)
     for (int k = 0; k < a.analyses[i].nsp; ++k) a.analyses[i].slot[k] = a.val_slot[a.analyses[i].sp[k]];
   e->analyses.assign(a.analyses, a.analyses + a.n_analyses);
-  size_t smem = (a.n_analyses > 0 ? sizeof(double) * a.n_vals * a.block_threads : 0) +
-                sizeof(int) * NUM_DELAY_REACTIONS * a.block_threads;
+  size_t smem = a.n_analyses > 0 ? sizeof(double) * a.n_vals * a.block_threads : 0;
   const size_t csr_bytes = sizeof(int) * max_edges;
   const size_t smem_cap = a.block_threads <= 224 ? 100000 : 200000;
   a.csr_in_smem = smem + csr_bytes <= smem_cap ? 1 : 0;

@@ -19,6 +19,7 @@ constexpr int kNP = NUM_PARAMS;
 constexpr int kMaxAnalyses = 8;
 constexpr int kStepThreads = 256;  // register kernel: one thread per cell, one CTA per set
 constexpr int kMaxCells = 65536;   // memory kernel: cells per set
+constexpr int64_t kMaxRegisterRing = 1 << 25;  // register kernel: elements of one set's history rings
 
 // Per-set status bits (also the public DENSE_SET_* values).
 enum : int {

@@ -252,8 +252,7 @@ extern "C" DENSE_API int dense_simulate_noalloc(const dense_run_desc* run, int n
                           reinterpret_cast<const int*>(base + o_status), s));
   a.csr_in_smem = 0;
   a.uniform_params = 0;  // parameters are laid out per cell here
-  NA_TRY(launch_step_fp64(a, reinterpret_cast<const int*>(base + o_list), num_sets,
-                          sizeof(int) * NUM_DELAY_REACTIONS * a.block_threads, s));
+  NA_TRY(launch_step_fp64(a, reinterpret_cast<const int*>(base + o_list), num_sets, 0, s));
 
   // ---- results to the caller's buffers
   size_t out_off = 0;

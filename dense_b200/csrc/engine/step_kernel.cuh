@@ -56,8 +56,6 @@ struct DeviceContext {
   const T* cur;            // this cell's lag-0 state [NS] (registers)
   const T* prm;            // parameters: shared row (pstride 1) or this cell's column (pstride n)
   int pstride;
-  const int* kd;           // truncated delays, kd[d * kd_stride] (shared)
-  int kd_stride;
   const int* S;            // DENSE ring sizes (shared)
   const int* mask;         // staged depth - 1 per species, -1 unstaged (shared)
   const int64_t* roff;     // ring offset per species (shared)
@@ -164,11 +162,198 @@ struct DeviceContext {
   // rates and delays are rejected when the batch is created.
   __device__ __forceinline__ T getRate(reaction_id r) const { return prm[r * pstride]; }
   __device__ __forceinline__ DelayArg<T> getDelay(delay_reaction_id d) const {
-    return DelayArg<T>{prm, pstride, static_cast<int>(d),
-                       kd ? kd[d * kd_stride] : static_cast<int>(prm[(kNR + d) * pstride])};
+    return DelayArg<T>{prm, pstride, static_cast<int>(d), static_cast<int>(prm[(kNR + d) * pstride])};
   }
   __device__ __forceinline__ T getCritVal(critspecie_id c) const { return prm[(kNR + kND + c) * pstride]; }
 };
+
+// ------------------------------------------------- register kernel reads
+// A history read resolved once per set (or cell): the lag it reads, 0 up to
+// the staged depth - 1, or a negative value for a read that the checked
+// rules flag (a delay DENSE would read out of bounds with, a lag the staging
+// does not keep, the row being written).
+constexpr int kReadLag0 = static_cast<int>(0x80000000u);     // row tables: an own read of lag 0
+constexpr int kReadChecked = static_cast<int>(0xC0000000u);  // a flagged read
+constexpr int kReadCheckBit = 0x40000000;
+
+// getCon(sp, k): lag (k - 1) mod S.
+__device__ __forceinline__ int resolve_own(int k, int S, int mask) {
+  if (k < 0 || k > S) return kReadChecked;
+  const int lag = k == 0 ? S - 1 : k - 1;
+  return lag > (mask > 0 ? mask : 0) ? kReadChecked : lag;
+}
+
+// calculateNeighborAvg(sp, k): lag k mod S.
+__device__ __forceinline__ int resolve_nbr(int k, int S, int mask) {
+  if (k < 0 || k > S) return kReadChecked;
+  const int lag = k == S ? 0 : k;
+  return (lag >= mask || (lag == S - 1 && S > 1)) ? kReadChecked : lag;
+}
+
+// What the reads of one step bring, by (delay reaction, species).  The
+// arrays are indexed by constants after inlining, so only the pairs a model
+// reads exist, in registers; has_* folds to a constant for every read that
+// does not hang on a condition in the model.
+template <typename T>
+struct Fetched {
+  T own[kND > 0 ? kND * kNS : 1], nbr[kND > 0 ? kND * kNS : 1];
+  bool has_own[kND > 0 ? kND * kNS : 1], has_nbr[kND > 0 ? kND * kNS : 1];
+  int seen;  // kReadCheckBit set once a flagged read was met
+};
+
+// The three passes over a model's rates in a step of the register kernel.
+enum ReadMode : int {
+  kFetch,    // make the delayed reads, keep what they bring (the rates themselves are dead code)
+  kUse,      // the rates, from what was fetched
+  kChecked,  // the rates with every read checked and flagged: steps with a flagged read
+};
+
+// Context of the register kernel.  Its delayed reads were the step's cost:
+// with the lag rules, 64-bit row arithmetic and their branches at each read,
+// a read took 60 instructions, and the branches kept every load next to its
+// use.  Measured on a 14-species gene network with 10 own and 2 neighbour
+// reads per cell-step: 1551 instructions per warp-step, 630 of them in the
+// own reads, 2.3 cycles per instruction waiting for loads; now 968 and 1.1
+// (4096 sets x 200 cells x 300 steps with Oscillation: 30.9 -> 16.6 ms a
+// run; a batch in FP32: 12.1 -> 7.1 ms; one set of 200 perturbed cells x
+// 1000 steps, whole call: 7.9 -> 5.6 ms).  To that end
+//  * everything that does not change from step to step is resolved before
+//    the loop (resolve_own, resolve_nbr).  kTable (one parameter row per
+//    set, so one lag per read and set): the element offset of each read's
+//    row is kept in a shared-memory table that the CTA's threads advance
+//    once per step, an entry each; else (a lag per cell) the row is formed
+//    from the lag, in 32 bits (the host gives sets with larger rings to the
+//    memory kernel);
+//  * the loads of a step are issued together before its rates (kFetch), so
+//    that their L2 latencies overlap;
+//  * flagged reads leave no branch in either pass: they only mark the step,
+//    and a marked step runs the checked pass instead.
+template <typename T, bool kTable, int kMode>
+struct RegContext {
+  const T* cur;            // this cell's lag-0 state [NS] (registers)
+  const T* prm;            // parameters: shared row (pstride 1) or this cell's column (pstride n)
+  int pstride;
+  const int* own_at;       // kTable: the step's row offsets [ND][NS] (shared), kReadLag0 or kReadChecked;
+  const int* nbr_at;       //   else the resolved reads [ND][NS] (registers)
+  const int* S;            // DENSE ring sizes (shared)
+  const int2* rows;        // {staged depth - 1 or -1, element offset of the ring} per species (shared)
+  const T* ring;           // this set's ring block
+  int step;                // Euler steps done: lag 0 sits in row step & mask
+  const int* nbr;          // this cell's neighbour ids (shared, or global for large lists)
+  int nnbr;
+  uint32_t nb01, nb23, nb45;  // the first six ids, 16 bits each
+  T rc;                    // RN(1 / nnbr), 0 without neighbours
+  int n_cells;
+  int cell;
+  int* err;
+  Fetched<T>* f;
+
+  __device__ __forceinline__ int row_at(specie_id sp, int lag) const {
+    const int2 r = rows[sp];
+    return ((step - lag) & r.x) * n_cells + r.y;
+  }
+
+  // DENSE's average over the neighbours: ascending ids, sum / count, NaN -> 0.
+  __device__ __forceinline__ T average(const T* row) const {
+    T sum = T(0);
+    if (nnbr <= kSmallCount) {
+      // absent neighbours' ids are 0: their loads stay in the row
+      const T v[6] = {row[nb01 & 0xFFFFu], row[nb01 >> 16], row[nb23 & 0xFFFFu],
+                      row[nb23 >> 16],     row[nb45 & 0xFFFFu], row[nb45 >> 16]};
+#pragma unroll
+      for (int e = 0; e < 6; ++e)
+        if (e < nnbr) sum += v[e];
+      if (small_count_operand(sum)) return div_by_small_count(sum, static_cast<T>(nnbr), rc);
+    } else {
+      for (int e = 0; e < nnbr; ++e) sum += row[nbr[e]];
+    }
+    const T avg = sum / static_cast<T>(nnbr);
+    return isnan(avg) ? T(0) : avg;
+  }
+
+  __device__ __forceinline__ T own_checked(specie_id sp, int k) const {
+    const int s = S[sp], m = rows[sp].x;
+    if (k < 0 || k > s + 1) *err |= kSetBadDelay;
+    const int lag = ((k - 1) % s + s) % s;
+    if (lag == 0) return cur[sp];
+    if (lag > m) {
+      *err |= kSetUnstagedLag;
+      return T(0);
+    }
+    return ring[row_at(sp, lag) + cell];
+  }
+
+  __device__ __forceinline__ T nbr_checked(specie_id sp, int k) const {
+    const int s = S[sp], m = rows[sp].x;
+    if (k < 0 || k > s) *err |= kSetBadDelay;
+    const int lag = (k % s + s) % s;
+    if (lag == s - 1 && s > 1) {
+      *err |= kSetOrderedReads;
+      return T(0);
+    }
+    if (lag >= m) {
+      *err |= kSetUnstagedLag;
+      return T(0);
+    }
+    return average(ring + row_at(sp, lag));
+  }
+
+  __device__ __forceinline__ T fetch_own(specie_id sp, int at) const {
+    f->seen |= at;
+    T v = cur[sp];
+    if (kTable) {
+      if (at >= 0) v = ring[at + cell];
+    } else {
+      if (at > 0) v = ring[row_at(sp, at) + cell];
+    }
+    return v;
+  }
+
+  __device__ __forceinline__ T fetch_nbr(specie_id sp, int at) const {
+    f->seen |= at;
+    if (at < 0) return T(0);
+    return average(ring + (kTable ? at : row_at(sp, at)));
+  }
+
+  __device__ __forceinline__ T getCon(specie_id sp) const { return cur[sp]; }
+  __device__ __forceinline__ T getCon(specie_id sp, int k) const { return own_checked(sp, k); }
+  __device__ __forceinline__ T getCon(specie_id sp, DelayArg<T> d) const {
+    if (kMode == kChecked) return own_checked(sp, d.k);
+    const int i = d.dr * kNS + sp;
+    if (kMode == kUse && f->has_own[i]) return f->own[i];
+    const T v = fetch_own(sp, own_at[i]);
+    f->own[i] = v;
+    f->has_own[i] = true;
+    return v;
+  }
+  __device__ __forceinline__ T calculateNeighborAvg(specie_id sp, int k = 0) const { return nbr_checked(sp, k); }
+  __device__ __forceinline__ T calculateNeighborAvg(specie_id sp, DelayArg<T> d) const {
+    if (kMode == kChecked) return nbr_checked(sp, d.k);
+    const int i = d.dr * kNS + sp;
+    if (kMode == kUse && f->has_nbr[i]) return f->nbr[i];
+    const T v = fetch_nbr(sp, nbr_at[i]);
+    f->nbr[i] = v;
+    f->has_nbr[i] = true;
+    return v;
+  }
+  __device__ __forceinline__ T getRate(reaction_id r) const { return prm[r * pstride]; }
+  __device__ __forceinline__ DelayArg<T> getDelay(delay_reaction_id d) const {
+    return DelayArg<T>{prm, pstride, static_cast<int>(d), static_cast<int>(prm[(kNR + d) * pstride])};
+  }
+  __device__ __forceinline__ T getCritVal(critspecie_id c) const { return prm[(kNR + kND + c) * pstride]; }
+
+  // the same context for another pass
+  template <int kOther>
+  __device__ __forceinline__ RegContext<T, kTable, kOther> as() const {
+    return RegContext<T, kTable, kOther>{cur, prm, pstride, own_at, nbr_at, S,    rows, ring, step,
+                                         nbr, nnbr, nb01,   nb23,   nb45,   rc,   n_cells, cell, err, f};
+  }
+};
+
+// The tables of RegContext fit in static shared memory up to this many
+// (delay reaction, species) pairs; models above it form their rows per read.
+constexpr int kPairs = kND * kNS;
+constexpr bool kRowTables = kPairs > 0 && kPairs <= 1024;
 
 // ------------------------------------------------------------ analyses
 // All per-cell analysis state is structure-of-arrays over the analysed
@@ -518,16 +703,24 @@ __device__ __forceinline__ bool analyses_sample(const StepArgs& a, double* anl, 
 // 16384), 256 threads with one CTA per SM above that.
 template <typename T, bool kKahan, int kThreads, int kMinBlocks, bool kUniform>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const StepArgs a, const int* set_list) {
-  // dynamic shared memory: sampled state [NS][blockDim] (doubles, only with
-  // analyses) | truncated delays [ND][blockDim] | the set's CSR lists
+  // dynamic shared memory: sampled state [n_vals][blockDim] (doubles, only
+  // with analyses) | the set's neighbour ids
   extern __shared__ double s_dyn[];
   double* s_vals = s_dyn;
-  __shared__ int s_S[kNS], s_mask[kNS];
-  __shared__ int64_t s_roff[kNS];
-  __shared__ T s_prm[kNP];
+  constexpr bool kTable = kUniform && kRowTables;
+  __shared__ int s_S[kNS];
+  __shared__ int2 s_rows[kNS];  // staged depth - 1 (-1: none), ring offset
+  __shared__ __align__(16) T s_prm[kNP];
   __shared__ int s_flags;
   __shared__ double s_samples[kMaxAnalyses];
-  __shared__ int s_olag[kND > 0 ? kND * kNS : 1], s_nlag[kND > 0 ? kND * kNS : 1];
+  // resolved reads (own, then neighbour); kTable: their row offsets of this
+  // step and the next, then the rows written, and the entries that advance
+  constexpr int kReads = kUniform ? 2 * kPairs : 0;
+  constexpr int kEntries = kTable ? 2 * kPairs + kNS : 0;
+  __shared__ int s_res[kReads > 0 ? kReads : 1];
+  __shared__ int s_at[2][kEntries > 0 ? kEntries : 1];
+  __shared__ unsigned short s_live[kEntries > 0 ? kEntries : 1];
+  __shared__ int s_n_live;
 
   const int set = set_list[blockIdx.x];
   const SetDesc& sd = a.sets[set];
@@ -539,17 +732,19 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
   const SetProgress pg = a.prog[set];
   if ((pg.status & (kSetDropped | kSetNotRunnable)) || pg.finalized) return;
 
-  const int pstride = sd.param_stride;
-  if (c < kNS) {
-    s_S[c] = sd.S[c];
-    s_mask[c] = sd.D[c] - 1;
-    s_roff[c] = sd.ring_off[c];
+  const int pstride = kUniform ? 0 : sd.param_stride;
+  for (int i = c; i < kNS; i += blk) {
+    s_S[i] = sd.S[i];
+    s_rows[i] = make_int2(sd.D[i] - 1, static_cast<int>(sd.ring_off[i]));
   }
   const T* P = static_cast<const T*>(a.params) + sd.param_base;
   if (pstride == 0) {
     for (int i = c; i < kNP; i += blk) s_prm[i] = P[i];
   }
-  if (c == 0) s_flags = 0;
+  if (c == 0) {
+    s_flags = 0;
+    s_n_live = 0;
+  }
   double* anl = a.anl + sd.anl_base;
   if (c < a.n_analyses) s_samples[c] = anl[a.analyses[c].off];
   __syncthreads();
@@ -559,27 +754,49 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
   // set's [NP][n] block (read through L1)
   const T* prm = pstride == 0 ? s_prm : P + cell;
   const int ps = pstride == 0 ? 1 : n;
+  int64_t step = pg.step;
+  int lres[kUniform || kPairs == 0 ? 1 : 2 * kPairs];  // !kUniform: this cell's reads
   if (kUniform) {
-    // lag tables of this set, with the exact lag rules of the checked path
-    for (int i = c; i < kND * kNS; i += blk) {
-      const int d = i / kNS, sp = i % kNS;
-      const int k = static_cast<int>(s_prm[kNR + d]);
-      const int S = s_S[sp], m = s_mask[sp];
-      int ol = -1, nl = -1;
-      if (k >= 0 && k <= S) {  // else: the checked path records a bad delay
-        ol = k - 1 < 0 ? S - 1 : k - 1;
-        if (ol != 0 && ol > m) ol = -1;
-        nl = k == S ? 0 : k;
-        if (nl >= m || nl == S - 1) nl = -1;
+    for (int i = c; i < kPairs; i += blk) {
+      const int k = static_cast<int>(s_prm[kNR + i / kNS]), sp = i % kNS;
+      s_res[i] = resolve_own(k, s_S[sp], s_rows[sp].x);
+      s_res[kPairs + i] = resolve_nbr(k, s_S[sp], s_rows[sp].x);
+    }
+  } else {
+#pragma unroll
+    for (int d = 0; d < kND; ++d) {
+      const int k = static_cast<int>(prm[(kNR + d) * ps]);
+#pragma unroll
+      for (int sp = 0; sp < kNS; ++sp) {
+        lres[d * kNS + sp] = resolve_own(k, s_S[sp], s_rows[sp].x);
+        lres[kPairs + d * kNS + sp] = resolve_nbr(k, s_S[sp], s_rows[sp].x);
       }
-      s_olag[i] = ol;
-      s_nlag[i] = nl;
     }
   }
-  int* s_kd = reinterpret_cast<int*>(s_dyn + (a.n_analyses > 0 ? a.n_vals * blk : 0));
-  int* s_csr = s_kd + kND * blk;
-#pragma unroll
-  for (int d = 0; d < kND; ++d) s_kd[d * blk + c] = static_cast<int>(prm[(kNR + d) * ps]);
+  // one entry of the row table: the offset of the row it names at step t
+  auto row_offset = [&](int e, int t) {
+    const bool write = e >= 2 * kPairs;
+    const int2 r = s_rows[write ? e - 2 * kPairs : e % kNS];
+    const int lag = write ? -1 : s_res[e];
+    return ((t - lag) & r.x) * n + r.y;
+  };
+  if (kTable) {
+    __syncthreads();
+    for (int e = c; e < kEntries; e += blk) {
+      int at = -1;
+      bool live;
+      if (e >= 2 * kPairs) {
+        live = s_rows[e - 2 * kPairs].x >= 0;
+      } else {
+        const int res = s_res[e];
+        live = e < kPairs ? res > 0 : res >= 0;
+        at = res < 0 ? kReadChecked : kReadLag0;
+      }
+      if (live) s_live[atomicAdd(&s_n_live, 1)] = static_cast<unsigned short>(e);
+      s_at[0][e] = s_at[1][e] = at;
+      if (live) s_at[step & 1][e] = row_offset(e, static_cast<int>(step));
+    }
+  }
 
   T cur[kNS];
   T comp[kNS];
@@ -593,8 +810,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
   const int nb0 = nbr_off[cell];
   const int nnbr = nbr_off[cell + 1] - nb0;
   const int* nbr = a.nbr_idx + nb0;
+  uint32_t nb[6];
+#pragma unroll
+  for (int e = 0; e < 6; ++e) nb[e] = e < nnbr ? static_cast<uint32_t>(nbr[e]) : 0u;
   if (a.csr_in_smem) {
     // the set's neighbour ids, [edges], in shared memory
+    int* s_csr = reinterpret_cast<int*>(s_dyn + (a.n_analyses > 0 ? a.n_vals * blk : 0));
     const int e0 = nbr_off[0], ne = nbr_off[n] - e0;
     for (int e = c; e < ne; e += blk) s_csr[e] = a.nbr_idx[e0 + e];
     nbr = s_csr + (nb0 - e0);
@@ -603,26 +824,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
 
   int err = 0;
   T* ring = static_cast<T*>(a.ring) + sd.ring_base;
-  int64_t step = pg.step;
-  // per-set constants of the history reads in registers (only the entries
-  // the model's reads use stay live); through shared memory they would be
-  // reloaded after every ring store
-  int64_t lroff[kNS];
-  int lmask[kNS];
-#pragma unroll
-  for (int sp = 0; sp < kNS; ++sp) {
-    lroff[sp] = s_roff[sp];
-    lmask[sp] = s_mask[sp];
-  }
-  int lolag[kND > 0 ? kND * kNS : 1], lnlag[kND > 0 ? kND * kNS : 1];
-#pragma unroll
-  for (int i = 0; i < kND * kNS; ++i) {
-    lolag[i] = s_olag[i];
-    lnlag[i] = s_nlag[i];
-  }
-  DeviceContext<T, kUniform> ctx{cur,  prm,    ps,   s_kd + cell, blk,    s_S,    lmask, lroff, ring,
-                                 static_cast<int>(step), nbr, nnbr, T(1) / static_cast<T>(nnbr), lolag, lnlag,
-                                 false, n, cell, &err};
+  const int n_live = kTable ? s_n_live : 0;
+  Fetched<T> fetched;
+  RegContext<T, kTable, kFetch> ctx{cur, prm, ps, kUniform ? s_res : lres, (kUniform ? s_res : lres) + kPairs, s_S,
+                                    s_rows, ring, static_cast<int>(step), nbr, nnbr, nb[0] | (nb[1] << 16),
+                                    nb[2] | (nb[3] << 16), nb[4] | (nb[5] << 16),
+                                    nnbr > 0 ? T(1) / static_cast<T>(nnbr) : T(0), n, cell, &err, &fetched};
 
   const T dt = static_cast<T>(a.dt);
   int chunk = pg.chunk;
@@ -631,6 +838,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
                             : chunk + a.chunk_count;
   double age = pg.age;
   bool dropped = false;
+  const int steps_per_chunk = sd.steps_per_chunk;
 
   for (; chunk < chunk_end; ++chunk) {
     // ---- analyses sample the state at `age` (measurement/base.ipp:4-9)
@@ -653,8 +861,19 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
     }
 
     // ---- (int)(interval/dt) Euler steps (determ.cpp:8-21, 77-88)
-    for (int s = 0; s < sd.steps_per_chunk; ++s) {
+    for (int s = 0; s < steps_per_chunk; ++s) {
       T nxt[kNS];
+      const int* at = s_at[ctx.step & 1];
+      if (kTable) {
+        ctx.own_at = at;
+        ctx.nbr_at = at + kPairs;
+        // the next step's rows
+        int* next = s_at[(ctx.step + 1) & 1];
+        for (int i = c; i < n_live; i += blk) {
+          const int e = s_live[i];
+          next[e] = row_offset(e, ctx.step + 1);
+        }
+      }
       if (active) {
         // DENSE evaluates every rate, then adds rate * delta reaction by
         // reaction (determ.cpp:58-72).  Each species' accumulator sees the
@@ -663,13 +882,25 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
         T dsp[kNS];
 #pragma unroll
         for (int sp = 0; sp < kNS; ++sp) dsp[sp] = T(0);
+        fetched.seen = 0;
+#pragma unroll
+        for (int i = 0; i < kPairs; ++i) fetched.has_own[i] = fetched.has_nbr[i] = false;
+#define REACTION(name) (void)reaction<name>::active_rate(ctx);
+#include "reactions_list.hpp"
+#undef REACTION
 #define REACTION(name)                                                        \
   {                                                                           \
-    const T rate_ = reaction<name>::active_rate(ctx);                         \
+    const T rate_ = reaction<name>::active_rate(rctx);                        \
     _Pragma("unroll") for (int j = 0; j < num_deltas_##name; j++)             \
         dsp[delta_ids_##name[j]] += rate_ * static_cast<T>(deltas_##name[j]); \
   }
+        if (__builtin_expect((fetched.seen & kReadCheckBit) == 0, 1)) {
+          const auto rctx = ctx.template as<kUse>();
 #include "reactions_list.hpp"
+        } else {
+          const auto rctx = ctx.template as<kChecked>();
+#include "reactions_list.hpp"
+        }
 #undef REACTION
 #pragma unroll
         for (int sp = 0; sp < kNS; ++sp) {
@@ -682,11 +913,15 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
             nxt[sp] = cur[sp] + dt * dsp[sp];
           }
         }
-        const int w = ctx.step + 1;
 #pragma unroll
         for (int sp = 0; sp < kNS; ++sp) {
-          const int m = s_mask[sp];
-          if (m >= 0) ring[s_roff[sp] + static_cast<int64_t>(w & m) * n + c] = nxt[sp];
+          if (kTable) {
+            const int w = at[2 * kPairs + sp];
+            if (w >= 0) ring[w + c] = nxt[sp];
+          } else {
+            const int2 r = s_rows[sp];
+            if (r.x >= 0) ring[((ctx.step + 1) & r.x) * n + r.y + c] = nxt[sp];
+          }
         }
       }
       __syncthreads();
@@ -696,7 +931,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
         for (int sp = 0; sp < kNS; ++sp) cur[sp] = nxt[sp];
       }
     }
-    step += sd.steps_per_chunk;
+    step += steps_per_chunk;
     age += a.interval;
   }
 
