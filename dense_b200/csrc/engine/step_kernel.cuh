@@ -1089,7 +1089,7 @@ __global__ void __launch_bounds__(256, 2) dense_step_mem_kernel(const StepArgs a
           const int ps = pstride == 0 ? 1 : n;
           const int nb0 = nbr_off[cell];
           const int cnt = nbr_off[cell + 1] - nb0;
-          DeviceContext<T, kUniform> ctx{cur,    prm,    ps,     nullptr, 0,      s_S,  s_mask, s_roff,
+          DeviceContext<T, kUniform> ctx{cur,    prm,    ps,     s_S,  s_mask, s_roff,
                                          ring,   st32,   a.nbr_idx + nb0, cnt,
                                          cnt < kRcTable ? s_rc[cnt] : T(1) / static_cast<T>(cnt),
                                          s_olag, s_nlag, ordered, n,      cell,   &err};
