@@ -669,7 +669,9 @@ __device__ __forceinline__ bool analyses_sample(const StepArgs& a, double* anl, 
       // of every analysed cell at every sample
       if (tid == 0) st[1] = age;
       if (!in_range) continue;
-      const long k = static_cast<long>(st[0]);
+      // the count as it was before this sample: thread 0 advances st[0] below
+      // while other warps may still be here
+      const long k = static_cast<long>(samples[ai]);
       if (k < A.range_steps) {
         const int m = A.cmax - A.cmin;
         double* vals_k = st + 2 + A.range_steps + static_cast<size_t>(k) * A.nsp * m;
