@@ -24,6 +24,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -100,15 +101,88 @@ void plan_levels(const dense_set_desc& in, bool ordered, SetPlan& plan) {
   plan.d.n_levels = n_levels;
 }
 
+// Device memory kept for the next batch.  cudaMalloc and cudaFree of more
+// than the driver's 2 MB chunks map and unmap memory: 0.3-1 ms and 0.3-3 ms
+// here (1 MB to 256 MB), as much as a small batch's run, and a search makes
+// and drops a batch per generation.  Allocations of up to kPoolKeep come
+// from a stream-ordered pool of the device that keeps at most kPoolKeep
+// (0.3 % of the GPU's memory) mapped once they are freed (1 us each then);
+// larger ones, and any the pool cannot serve, are plain cudaMalloc.  The
+// pool is the driver's own object: calls from several threads are safe, and
+// an allocation is freed only after the device has been synchronised, so no
+// stream can still use it.
+constexpr size_t kPoolKeep = size_t(512) << 20;
+
+struct DevicePool {
+  cudaMemPool_t pool = nullptr;
+  cudaStream_t stream = nullptr;  // orders the pool's allocations and frees
+};
+
+DevicePool device_pool(int device) {
+  constexpr int kMaxDevices = 64;
+  static std::mutex mu;
+  static DevicePool pools[kMaxDevices];
+  static bool tried[kMaxDevices] = {};
+  if (device < 0 || device >= kMaxDevices) return {};
+  std::lock_guard<std::mutex> lock(mu);
+  if (!tried[device]) {
+    tried[device] = true;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    DevicePool made;
+    uint64_t keep = kPoolKeep;
+    if (cudaMemPoolCreate(&made.pool, &props) == cudaSuccess &&
+        cudaMemPoolSetAttribute(made.pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess &&
+        cudaStreamCreateWithFlags(&made.stream, cudaStreamNonBlocking) == cudaSuccess)
+      pools[device] = made;
+    else
+      cudaGetLastError();
+  }
+  return pools[device];
+}
+
 struct DeviceBuffer {
   void* p = nullptr;
   size_t bytes = 0;
+  bool owned = true;   // false: a part of another buffer
+  cudaStream_t pool_stream = nullptr;  // set: from the device's pool
+  DeviceBuffer() = default;
+  DeviceBuffer(const DeviceBuffer&) = delete;
+  DeviceBuffer& operator=(const DeviceBuffer&) = delete;
   ~DeviceBuffer() {
-    if (p) cudaFree(p);
+    if (!p || !owned) return;
+    if (pool_stream) {
+      cudaDeviceSynchronize();
+      cudaFreeAsync(p, pool_stream);
+    } else {
+      cudaFree(p);
+    }
+  }
+  void view(void* at, size_t n) {
+    p = at;
+    bytes = n;
+    owned = false;
   }
   int alloc(size_t n) {
     bytes = n;
     if (n == 0) n = 16;
+    int device = 0;
+    if (n <= kPoolKeep && cudaGetDevice(&device) == cudaSuccess) {
+      const DevicePool pool = device_pool(device);
+      if (pool.pool) {
+        // (synchronised, so usable on every stream)
+        if (cudaMallocFromPoolAsync(&p, n, pool.pool, pool.stream) == cudaSuccess &&
+            cudaStreamSynchronize(pool.stream) == cudaSuccess) {
+          pool_stream = pool.stream;
+          return DENSE_OK;
+        }
+        p = nullptr;
+        cudaGetLastError();
+        cudaMemPoolTrimTo(pool.pool, 0);
+      }
+    }
     cudaError_t e = cudaMalloc(&p, n);
     if (e != cudaSuccess) {
       p = nullptr;
@@ -133,6 +207,8 @@ struct dense_engine {
   std::vector<SetDesc> sets;
   std::vector<AnalysisDesc> analyses;
   std::vector<int> init_status;
+  // one allocation holds every buffer below
+  DeviceBuffer d_all;
   DeviceBuffer d_sets, d_prog, d_params, d_nbr_off, d_nbr_idx, d_state, d_ring, d_anl, d_init_conc,
       d_init_status, d_lists, d_lvl_off, d_lvl_cells, d_wave_rec;
   int n_reg = 0, n_mem = 0;  // sets run by the register / memory kernels (d_lists: reg then mem)
@@ -143,16 +219,19 @@ struct dense_engine {
   std::vector<std::array<int, 5>> mem_groups;
   std::map<int, cudaGraphExec_t> graphs;
   // the kernel launches of one run (register kernel, one per memory- or
-  // wave-kernel group) fork onto side streams of their own so that they run
+  // wave-kernel group) fork onto streams of their own so that they run
   // concurrently; launch k goes to side[k], whose priority ranks the
   // group's longest set (the block scheduler starts the CTAs of
-  // higher-priority streams first)
+  // higher-priority streams first).  side[0] is the engine's own stream
+  // (making and destroying a stream costs 55 us each, and most batches have
+  // one launch).
   std::vector<cudaStream_t> side;
   std::vector<cudaEvent_t> ev_join;
   cudaEvent_t ev_fork = nullptr;
   ~dense_engine() {
     for (auto& g : graphs) cudaGraphExecDestroy(g.second);
-    for (auto& x : side) cudaStreamDestroy(x);
+    for (auto& x : side)
+      if (x != stream) cudaStreamDestroy(x);
     for (auto& x : ev_join) cudaEventDestroy(x);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (stream) cudaStreamDestroy(stream);
@@ -169,14 +248,14 @@ int next_pow2(int x) {
 }
 
 // Input checks of one set (CSR tissue, sizes, hints).
-int check_set(const dense_set_desc& in, const std::string& where) {
+int check_set(const dense_set_desc& in, const std::string& where, bool tissue = true) {
   if (in.num_cells <= 0 || in.num_cells > kMaxCells)
     return fail(DENSE_ERR_UNSUPPORTED, where + "1.." + std::to_string(kMaxCells) + " cells per set are supported");
   if (!in.nbr_offsets || !in.nbr_ids || !in.set_params) return fail(DENSE_ERR_INVALID, where + "null input");
   if (!(in.duration >= 0.0)) return fail(DENSE_ERR_INVALID, where + "negative duration");
   const int n = in.num_cells;
   if (in.nbr_offsets[0] != 0) return fail(DENSE_ERR_INVALID, where + "CSR offsets must start at 0");
-  for (int c = 0; c < n; ++c) {
+  for (int c = 0; tissue && c < n; ++c) {
     if (in.nbr_offsets[c + 1] < in.nbr_offsets[c]) return fail(DENSE_ERR_INVALID, where + "CSR offsets decrease");
     for (int k = in.nbr_offsets[c]; k < in.nbr_offsets[c + 1]; ++k) {
       const int v = in.nbr_ids[k];
@@ -510,6 +589,9 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
   // ---- sets
   std::vector<double> params_all, conc_all(static_cast<size_t>(num_sets) * NUM_SPECIES, 0.0);
   std::vector<int> off_all, idx_all;
+  // sets given with the same neighbour arrays share one copy on the device
+  // (and its checks): the tissue of a parameter search is one for all sets
+  std::map<std::pair<const int*, const int*>, std::pair<int, int64_t>> tissues;  // -> (cells, nbr_base)
   int64_t cells_total = 0, ring_total = 0;
   int max_cells = 0, max_edges = 0;
   std::vector<int> reg_list, mem_list, mem_block_of, mem_smem_of, mem_kind_of, lvl_off_all, lvl_cells_all;
@@ -520,8 +602,10 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
   for (int s = 0; s < num_sets; ++s) {
     const dense_set_desc& in = in_sets[s];
     const std::string where = "set " + std::to_string(s) + ": ";
+    const auto known = tissues.find({in.nbr_offsets, in.nbr_ids});
+    const bool shared_tissue = known != tissues.end() && known->second.first == in.num_cells;
     {
-      const int rc = check_set(in, where);
+      const int rc = check_set(in, where, !shared_tissue);
       if (rc != DENSE_OK) return rc;
     }
     const int n = in.num_cells;
@@ -535,13 +619,18 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
     d.steps_per_chunk = steps_per_chunk;
     d.param_base = static_cast<int64_t>(params_all.size());
     d.cell_base = cells_total;
-    d.nbr_base = static_cast<int64_t>(off_all.size());
     d.ring_base = ring_total;
     d.anl_base = anl_block * s;
     e->anl_block = anl_block;
-    const int e0 = static_cast<int>(idx_all.size());
-    for (int c = 0; c <= n; ++c) off_all.push_back(e0 + in.nbr_offsets[c]);
-    idx_all.insert(idx_all.end(), in.nbr_ids, in.nbr_ids + in.nbr_offsets[n]);
+    if (shared_tissue) {
+      d.nbr_base = known->second.second;
+    } else {
+      d.nbr_base = static_cast<int64_t>(off_all.size());
+      tissues[{in.nbr_offsets, in.nbr_ids}] = {n, d.nbr_base};
+      const int e0 = static_cast<int>(idx_all.size());
+      for (int c = 0; c <= n; ++c) off_all.push_back(e0 + in.nbr_offsets[c]);
+      idx_all.insert(idx_all.end(), in.nbr_ids, in.nbr_ids + in.nbr_offsets[n]);
+    }
     params_all.insert(params_all.end(), cp.begin(), cp.end());
     if (in.init_conc)
       for (int sp = 0; sp < NUM_SPECIES; ++sp) conc_all[static_cast<size_t>(s) * NUM_SPECIES + sp] = in.init_conc[sp];
@@ -582,24 +671,37 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
     e->sets[s] = d;
   }
 
-  // ---- device buffers
-  CUDA_TRY(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
+  // ---- device buffers: what the host writes first, in one upload
   const size_t tsz = run->precision == DENSE_FP64 ? sizeof(double) : sizeof(float);
   int rc;
-  if ((rc = e->d_sets.alloc(sizeof(SetDesc) * num_sets))) return rc;
-  if ((rc = e->d_prog.alloc(sizeof(SetProgress) * num_sets))) return rc;
-  if ((rc = e->d_params.alloc(tsz * params_all.size()))) return rc;
-  if ((rc = e->d_nbr_off.alloc(sizeof(int) * off_all.size()))) return rc;
-  if ((rc = e->d_nbr_idx.alloc(sizeof(int) * idx_all.size()))) return rc;
-  if ((rc = e->d_state.alloc(tsz * 2 * NUM_SPECIES * cells_total))) return rc;
-  if ((rc = e->d_ring.alloc(tsz * ring_total))) return rc;
-  if ((rc = e->d_anl.alloc(sizeof(double) * anl_block * num_sets))) return rc;
-  if ((rc = e->d_init_conc.alloc(sizeof(double) * conc_all.size()))) return rc;
-  if ((rc = e->d_init_status.alloc(sizeof(int) * num_sets))) return rc;
-  if ((rc = e->d_lists.alloc(sizeof(int) * num_sets))) return rc;
-  if ((rc = e->d_lvl_off.alloc(sizeof(int) * std::max<size_t>(1, lvl_off_all.size())))) return rc;
-  if ((rc = e->d_lvl_cells.alloc(sizeof(int) * lvl_cells_all.size()))) return rc;
-  if ((rc = e->d_wave_rec.alloc(sizeof(uint16_t) * rec_all.size()))) return rc;
+  if (mem_list.empty()) std::vector<int>().swap(lvl_cells_all);  // only the memory kernel reads cells in level order
+  struct Part {
+    DeviceBuffer* b;
+    size_t bytes, at;
+  };
+  Part parts[] = {{&e->d_sets, sizeof(SetDesc) * num_sets, 0},
+                  {&e->d_params, tsz * params_all.size(), 0},
+                  {&e->d_nbr_off, sizeof(int) * off_all.size(), 0},
+                  {&e->d_nbr_idx, sizeof(int) * idx_all.size(), 0},
+                  {&e->d_init_conc, sizeof(double) * conc_all.size(), 0},
+                  {&e->d_init_status, sizeof(int) * num_sets, 0},
+                  {&e->d_lists, sizeof(int) * num_sets, 0},
+                  {&e->d_lvl_off, sizeof(int) * lvl_off_all.size(), 0},
+                  {&e->d_lvl_cells, sizeof(int) * lvl_cells_all.size(), 0},
+                  {&e->d_wave_rec, sizeof(uint16_t) * rec_all.size(), 0},
+                  {&e->d_prog, sizeof(SetProgress) * num_sets, 0},
+                  {&e->d_state, tsz * 2 * NUM_SPECIES * cells_total, 0},
+                  {&e->d_ring, tsz * ring_total, 0},
+                  {&e->d_anl, sizeof(double) * anl_block * num_sets, 0}};
+  constexpr int kUploads = 10;  // the first parts
+  size_t total = 0, upload = 0;
+  for (int i = 0; i < static_cast<int>(sizeof parts / sizeof parts[0]); ++i) {
+    parts[i].at = total;
+    total += (std::max<size_t>(parts[i].bytes, 16) + 255) & ~size_t(255);
+    if (i + 1 == kUploads) upload = total;
+  }
+  if ((rc = e->d_all.alloc(total))) return rc;
+  for (Part& x : parts) x.b->view(static_cast<char*>(e->d_all.p) + x.at, x.bytes);
   e->n_reg = static_cast<int>(reg_list.size());
   e->n_mem = static_cast<int>(mem_list.size());
   {
@@ -627,18 +729,6 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
         e->mem_groups.push_back({key[0], key[2], key[1], static_cast<int>(k), 0});
       e->mem_groups.back()[4]++;
     }
-    std::vector<int> lists(reg_list);
-    lists.insert(lists.end(), mem_list.begin(), mem_list.end());
-    CUDA_TRY(cudaMemcpyAsync(e->d_lists.p, lists.data(), sizeof(int) * num_sets, cudaMemcpyHostToDevice, e->stream));
-    if (!lvl_off_all.empty())
-      CUDA_TRY(cudaMemcpyAsync(e->d_lvl_off.p, lvl_off_all.data(), sizeof(int) * lvl_off_all.size(),
-                               cudaMemcpyHostToDevice, e->stream));
-    CUDA_TRY(cudaMemcpyAsync(e->d_lvl_cells.p, lvl_cells_all.data(), sizeof(int) * lvl_cells_all.size(),
-                             cudaMemcpyHostToDevice, e->stream));
-    if (!rec_all.empty())
-      CUDA_TRY(cudaMemcpyAsync(e->d_wave_rec.p, rec_all.data(), sizeof(uint16_t) * rec_all.size(),
-                               cudaMemcpyHostToDevice, e->stream));
-    CUDA_TRY(cudaStreamSynchronize(e->stream));
   }
   {
     // one side stream per launch, prioritised by the group's longest set in
@@ -674,26 +764,29 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
       cudaStream_t x;
       cudaEvent_t ev;
       CUDA_TRY(cudaStreamCreateWithPriority(&x, cudaStreamNonBlocking, prio[i]));
+      if (i == 0) e->stream = x;
       e->side.push_back(x);
       CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
       e->ev_join.push_back(ev);
     }
   }
-  CUDA_TRY(cudaMemcpyAsync(e->d_sets.p, e->sets.data(), sizeof(SetDesc) * num_sets, cudaMemcpyHostToDevice, e->stream));
-  std::vector<float> params_f;
-  if (run->precision == DENSE_FP64) {
-    CUDA_TRY(cudaMemcpyAsync(e->d_params.p, params_all.data(), sizeof(double) * params_all.size(),
-                             cudaMemcpyHostToDevice, e->stream));
-  } else {
-    params_f.assign(params_all.begin(), params_all.end());
-    CUDA_TRY(cudaMemcpyAsync(e->d_params.p, params_f.data(), sizeof(float) * params_f.size(),
-                             cudaMemcpyHostToDevice, e->stream));
+  {
+    // staged in one block and copied at once
+    std::vector<int> lists(reg_list);
+    lists.insert(lists.end(), mem_list.begin(), mem_list.end());
+    std::vector<float> params_f;
+    if (run->precision != DENSE_FP64) params_f.assign(params_all.begin(), params_all.end());
+    const void* const from[kUploads] = {e->sets.data(),
+                                        run->precision == DENSE_FP64 ? static_cast<const void*>(params_all.data())
+                                                                     : params_f.data(),
+                                        off_all.data(), idx_all.data(), conc_all.data(), e->init_status.data(),
+                                        lists.data(), lvl_off_all.data(), lvl_cells_all.data(), rec_all.data()};
+    std::vector<unsigned char> staged(upload);
+    for (int i = 0; i < kUploads; ++i)
+      if (parts[i].bytes > 0) std::memcpy(staged.data() + parts[i].at, from[i], parts[i].bytes);
+    CUDA_TRY(cudaMemcpyAsync(e->d_all.p, staged.data(), upload, cudaMemcpyHostToDevice, e->stream));
+    CUDA_TRY(cudaStreamSynchronize(e->stream));
   }
-  CUDA_TRY(cudaMemcpyAsync(e->d_nbr_off.p, off_all.data(), sizeof(int) * off_all.size(), cudaMemcpyHostToDevice, e->stream));
-  if (!idx_all.empty())
-    CUDA_TRY(cudaMemcpyAsync(e->d_nbr_idx.p, idx_all.data(), sizeof(int) * idx_all.size(), cudaMemcpyHostToDevice, e->stream));
-  CUDA_TRY(cudaMemcpyAsync(e->d_init_conc.p, conc_all.data(), sizeof(double) * conc_all.size(), cudaMemcpyHostToDevice, e->stream));
-  CUDA_TRY(cudaMemcpyAsync(e->d_init_status.p, e->init_status.data(), sizeof(int) * num_sets, cudaMemcpyHostToDevice, e->stream));
   e->device_bytes = static_cast<int64_t>(e->d_sets.bytes + e->d_prog.bytes + e->d_params.bytes + e->d_nbr_off.bytes +
                                          e->d_nbr_idx.bytes + e->d_state.bytes + e->d_ring.bytes + e->d_anl.bytes +
                                          e->d_init_conc.bytes + e->d_init_status.bytes);
@@ -769,11 +862,11 @@ static cudaError_t launch_all(dense_engine* e, const StepArgs& a, cudaStream_t s
   int k = 0;  // launches issued so far
   auto stream_for = [&](cudaStream_t& st) -> cudaError_t {
     st = e->side[k];
-    return cudaStreamWaitEvent(st, e->ev_fork, 0);
+    return st == s ? cudaSuccess : cudaStreamWaitEvent(st, e->ev_fork, 0);
   };
   auto join = [&](cudaStream_t st) -> cudaError_t {
-    cudaError_t rj = cudaEventRecord(e->ev_join[k], st);
-    if (rj == cudaSuccess) rj = cudaStreamWaitEvent(s, e->ev_join[k], 0);
+    cudaError_t rj = st == s ? cudaSuccess : cudaEventRecord(e->ev_join[k], st);
+    if (st != s && rj == cudaSuccess) rj = cudaStreamWaitEvent(s, e->ev_join[k], 0);
     ++k;
     return rj;
   };

