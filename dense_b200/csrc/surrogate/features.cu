@@ -7,6 +7,8 @@
 
 #include "dense_b200_surrogate.h"
 
+#include <cooperative_groups.h>
+
 #include <cmath>
 #include <cstdint>
 
@@ -18,8 +20,13 @@
 
 namespace {
 
-constexpr int kSyncThreads = 256;
+constexpr int kSyncThreads = 512;
 constexpr int kMaxSyncCells = 1024;
+constexpr int kSyncGroups = kSyncThreads / 32;
+constexpr int kSyncInv = 64;
+// Bytes of the trajectories in flight (two CTAs per SM) that the 126 MB L2
+// keeps between the kernel's two passes.
+constexpr int64_t kSyncL2 = int64_t(80) << 20;
 
 __device__ __forceinline__ double quiet_nan() { return __longlong_as_double(0x7FF8000000000000LL); }
 
@@ -34,76 +41,171 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   return t;
 }
 
-__device__ __forceinline__ double block_max(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) red[w] = v;
-  __syncthreads();
-  double t = 0.0;
-  for (int i = 0; i < static_cast<int>(blockDim.x >> 5); ++i) t = fmax(t, red[i]);
-  return t;
-}
-
 // Mean pairwise Pearson correlation across the cells of each set's
 // trajectory X[set][t][cell] (t < counts[set]; cells contiguous), cells
 // with a constant trace left out:
 //   sum_{i != j} <z_i, z_j> = |sum_i z_i|^2 - n  for unit, zero-mean z_i,
-// divided by n (n - 1); NaN when fewer than two cells remain.  One CTA per
-// set: per cell the mean and the norm (two passes over the samples, in
-// sample order), then per sample the sum over cells of z (a warp per
-// sample, lanes over cells) and the sum of its squares.
-__global__ void __launch_bounds__(kSyncThreads) synchrony_kernel(const double* __restrict__ X, int64_t set_stride,
-                                                                 int64_t sample_stride, int cells,
-                                                                 const int* __restrict__ counts,
-                                                                 double* __restrict__ out) {
-  __shared__ double mean[kMaxSyncCells], scale[kMaxSyncCells];
-  __shared__ double red[kSyncThreads / 32];
-  const int set = blockIdx.x;
-  const int T = counts[set];
-  const double* x = X + set * set_stride;
-  double top = 0.0, nan_seen = 0.0;
-  for (int c = threadIdx.x; c < cells; c += blockDim.x) {
-    double s = 0.0;
-    for (int t = 0; t < T; ++t) {
-      const double v = x[t * sample_stride + c];
-      s += v;
-      top = fmax(top, fabs(v));
-      if (isnan(v)) nan_seen = 1.0;
-    }
-    mean[c] = T > 0 ? s / T : 0.0;
+// divided by n (n - 1); NaN when fewer than two cells remain.
+//
+// Two passes over the samples: the cells' means and squared deviations
+// (blocks of eight samples two-pass in registers, joined by the pairwise
+// update of Chan, Golub and LeVeque, 1983, which keeps the two-pass
+// accuracy), then per sample the sum of z over the cells.  A set's samples
+// (600 x 200 doubles: 0.96 MB) are shared by a cluster of CTAs, as many as
+// keep the sets in flight within the L2 cache, so that the second pass does
+// not go back to HBM; the CTAs' statistics meet in distributed shared
+// memory, joined in rank order.  1500 sets x 600 x 200, 1.44 GB: 0.54 ms (2.7 TB/s
+// from HBM, 5.4 TB/s read), bound by issue (45 %) and the barriers between
+// the passes; with one CTA per set and three passes, every one from HBM,
+// 1.17 ms.  (Slices of the samples kept in shared memory, 8 or 16 CTAs a
+// set, took 1.6 ms: the exchange and the reductions of so many CTAs cost
+// more than the reads they save.)
+struct CellStats {
+  double n, mean, m2;
+  __device__ __forceinline__ void join(double bn, double bmean, double bm2) {
+    if (bn <= 0.0) return;
+    const double total = n + bn, w = bn / total, d = bmean - mean;
+    mean += d * w;
+    m2 += bm2 + d * d * (n * w);
+    n = total;
   }
-  top = block_max(top, red);
-  // a NaN sample makes the largest magnitude NaN, and then no cell counts
-  if (block_max(nan_seen, red) > 0.0) top = quiet_nan();
-  double n_ok = 0.0;
-  for (int c = threadIdx.x; c < cells; c += blockDim.x) {
-    const double m = mean[c];
-    double q = 0.0;
-    for (int t = 0; t < T; ++t) {
-      const double d = x[t * sample_stride + c] - m;
-      q += d * d;
+};
+
+__global__ void __launch_bounds__(kSyncThreads, 2) synchrony_kernel(const double* __restrict__ X, int64_t set_stride,
+                                                                    int64_t sample_stride, int cells,
+                                                                    const int* __restrict__ counts,
+                                                                    double* __restrict__ out) {
+  __shared__ double red[kSyncThreads / 32];
+  extern __shared__ double sy_dyn[];
+  __shared__ double s_n[kSyncGroups];                       // samples of each thread group
+  const int threads = blockDim.x, wide = max(threads, cells);
+  double* s_mean = sy_dyn;                                  // the groups' statistics, [group][cell]
+  double* s_m2 = s_mean + wide;
+  double* r_mean = s_m2 + wide;                             // this rank's, read by the others
+  double* r_m2 = r_mean + cells;
+  double* centre = r_m2 + cells;                            // the cells' means over every rank
+  __shared__ int share_top;
+  __shared__ double share_sq;
+  __shared__ double s_inv[kSyncInv];                        // 1 / (k + 1)
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ranks = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
+  const int set = blockIdx.x / ranks;
+  const int T = counts[set];
+  const int per = T > 0 ? (T + ranks - 1) / ranks : 0;
+  const int t0 = min(T, rank * per), rows = max(0, min(T, t0 + per) - t0);
+  const double* x = X + set * set_stride + t0 * sample_stride;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int warps = threads >> 5;
+
+  // pass 1: rows dealt over thread groups of `width` threads, eight
+  // neighbouring rows at a time
+  int width = 32;
+  while (width < cells && width < threads) width *= 2;
+  const int groups = threads / width, grp = tid / width, first = tid % width;
+  // largest magnitude, to the 20 mantissa bits of its upper word (it only
+  // scales the test for constant traces); infinities and NaN lie above all
+  int top = 0;
+  auto magnitude = [&](double v) { top = max(top, __double2hiint(v) & 0x7fffffff); };
+  for (int i = tid; i < kSyncInv; i += threads) s_inv[i] = 1.0 / (i + 1);
+  if (tid == 0) share_top = 0;
+  __syncthreads();
+  for (int c = first; c < cells; c += width) {
+    const double* p = x + c + static_cast<int64_t>(grp) * 8 * sample_stride;
+    const int64_t hop = static_cast<int64_t>(groups) * 8 * sample_stride;
+    double mean = 0.0, m2 = 0.0;
+    int t = grp * 8, k = 0;  // k whole blocks joined
+    for (; t + 8 <= rows; t += groups * 8, p += hop, ++k) {
+      double v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = p[j * sample_stride];
+      const double m = (((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]))) * 0.125;
+      double q0 = 0.0, q1 = 0.0;
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) {
+        magnitude(v[j]);
+        magnitude(v[j + 1]);
+        const double d0 = v[j] - m, d1 = v[j + 1] - m;
+        q0 += d0 * d0;
+        q1 += d1 * d1;
+      }
+      // CellStats::join of equal blocks: k blocks and one more
+      const double w = k < kSyncInv ? s_inv[k] : 1.0 / (k + 1), d = m - mean;
+      mean += d * w;
+      m2 += (q0 + q1) + d * d * (8.0 * k * w);
     }
-    const double nrm = sqrt(q);
-    const bool ok = nrm > 1e-12 * (1.0 + top);
-    scale[c] = ok ? nrm : 0.0;
+    CellStats st{8.0 * k, mean, m2};
+    for (int j = 0; t + j < rows && j < 8; ++j) {
+      const double v = p[j * sample_stride];
+      magnitude(v);
+      st.join(1.0, v, 0.0);
+    }
+    s_mean[grp * width + c] = st.mean;  // (one group when cells > width)
+    s_m2[grp * width + c] = st.m2;
+    if (c == 0) s_n[grp] = st.n;
+  }
+  __syncthreads();
+  for (int c = tid; c < cells; c += threads) {
+    CellStats st{0.0, 0.0, 0.0};
+    for (int g = 0; g < groups; ++g) st.join(s_n[g], s_mean[g * width + c], s_m2[g * width + c]);
+    r_mean[c] = st.mean;
+    r_m2[c] = st.m2;
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) atomicMax(&share_top, top);
+  cluster.sync();
+  for (int k = 0; k < ranks; ++k) top = max(top, *cluster.map_shared_rank(&share_top, k));
+  // with an infinite or NaN sample no cell counts (the comparison fails)
+  const double largest = __hiloint2double(top, 0);
+  double n_ok = 0.0;
+  for (int c = tid; c < cells; c += threads) {
+    CellStats st{0.0, 0.0, 0.0};
+    for (int k = 0; k < ranks; ++k) {
+      const int rk = max(0, min(T, k * per + per) - min(T, k * per));
+      st.join(rk, cluster.map_shared_rank(r_mean, k)[c], cluster.map_shared_rank(r_m2, k)[c]);
+    }
+    const double nrm = sqrt(st.m2);
+    const bool ok = nrm > 1e-12 * (1.0 + largest);
+    centre[c] = st.mean;
+    s_mean[c] = ok ? nrm : 0.0;  // the groups' statistics are done with: now the norms (0: left out)
+    s_m2[c] = ok ? 1.0 / nrm : 0.0;  // and their reciprocals
     n_ok += ok ? 1.0 : 0.0;
   }
-  const double n = block_sum(n_ok, red);
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const double n = block_sum(n_ok, red);  // (its barriers also publish the norms)
+
+  // pass 2: a warp per four samples; the quotient from the reciprocal with
+  // one FMA correction (its error stays below one ulp of the division's)
   double s2 = 0.0;
-  for (int t = warp; t < T; t += warps) {
-    double s = 0.0;
+  for (int t = 4 * warp; t < rows; t += 4 * warps) {
+    const int live = min(4, rows - t);
+    const double* p = x + static_cast<int64_t>(t) * sample_stride;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
     for (int c = lane; c < cells; c += 32) {
-      const double nrm = scale[c];
-      if (nrm > 0.0) s += (x[t * sample_stride + c] - mean[c]) / nrm;
+      double v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = p[(j < live ? j : 0) * sample_stride + c];
+      const double m = centre[c], nrm = s_mean[c], inv = s_m2[c];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const double d = v[j] - m, q = d * inv;
+        s[j] += __fma_rn(__fma_rn(-q, nrm, d), inv, q);
+      }
     }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    s2 += s * s;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+      if (j < live) s2 += s[j] * s[j];
+    }
   }
-  const double total = block_sum(lane == 0 ? s2 : 0.0, red);
-  if (threadIdx.x == 0) out[set] = n >= 2.0 ? (total - n) / (n * (n - 1.0)) : quiet_nan();
+  const double mine = block_sum(lane == 0 ? s2 : 0.0, red);
+  if (tid == 0) share_sq = mine;
+  cluster.sync();
+  if (rank == 0 && tid == 0) {
+    double total = 0.0;
+    for (int k = 0; k < ranks; ++k) total += *cluster.map_shared_rank(&share_sq, k);
+    out[set] = n >= 2.0 ? (total - n) / (n * (n - 1.0)) : quiet_nan();
+  }
+  cluster.sync();  // every rank's shared memory stays until rank 0 has read it
 }
 
 // Network inputs of candidates P[r][ldp] (float64 parameters):
@@ -174,9 +276,32 @@ FEATURES_API int dense_features_synchrony(const double* X, int64_t set_stride, i
                                           const int* counts, int n_sets, double* out, void* stream) {
   if (n_sets < 0 || cells < 0 || cells > kMaxSyncCells) return 1;
   if (n_sets == 0) return 0;
-  synchrony_kernel<<<n_sets, kSyncThreads, 0, static_cast<cudaStream_t>(stream)>>>(X, set_stride, sample_stride, cells,
-                                                                                  counts, out);
-  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+  // the most samples a set can have in this layout (unknown, taken as few,
+  // when the sets are not the outer dimension)
+  const int64_t cap = sample_stride > 0 && set_stride >= sample_stride ? set_stride / sample_stride : 0;
+  int ranks = 1;
+  while (ranks < 8 && (296 / ranks * cap * cells * 8 > kSyncL2 ||
+                       (static_cast<int64_t>(n_sets) * ranks < 296 && cap / ranks > 32)))
+    ranks *= 2;
+  // threads by a CTA's share of a set: the fixed part (reductions, exchange)
+  // of 512 threads outweighs small sets (1500 sets x 50 x 20: 53 us with 512,
+  // 32 us with 128; 700 sets x 100 x 200 with 256: 62 us either way; the
+  // largest shares want all 512: 0.54 ms against 0.64 ms with 256)
+  const int64_t share = cap * cells / ranks;
+  const int threads = cap == 0 || share >= 16384 ? kSyncThreads : (share >= 4096 ? 256 : 128);
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = ranks;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(n_sets * ranks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = sizeof(double) * (2 * (threads > cells ? threads : cells) + 3 * cells);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, synchrony_kernel, X, set_stride, sample_stride, cells, counts, out);
+  return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
 FEATURES_API int dense_features_encode(const double* P, int ldp, int n, const int* idx, const double* tmpl, int k,
