@@ -298,11 +298,12 @@ def predicted_score(pred):
 
 def score_candidates(net, P, chunk=1 << 20, spread=SPREAD, batch=65536):
     """predicted_score(net.predict(encode(P))) on the GPU: per chunk of
-    candidates one host-to-device copy of their parameters, then the
-    encoding, every network of the ensemble (`net` a Surrogate, or one MLP)
-    and the score in the surrogate library's kernels; float64 numpy array."""
+    candidates one host-to-device copy of their parameters, then one launch
+    for the encoding, every network of the ensemble (`net` a Surrogate, or
+    one MLP) and the score; float64 numpy array.  (`batch`: rows at a time
+    for an ensemble of more than MAX_NETS networks.)"""
     import torch
-    from .surrogate import IN_PAD
+    from .surrogate import IN_PAD, MAX_NETS
     nets = getattr(net, "nets", None) or [net]
     n_out = nets[0].n_out
     mu = getattr(net, "mu", np.zeros(n_out, np.float32))
@@ -312,22 +313,27 @@ def score_candidates(net, P, chunk=1 << 20, spread=SPREAD, batch=65536):
     idx = active_params()
     idx_d = torch.as_tensor(idx.astype(np.int32), device=dev)
     t_d = torch.as_tensor(template()[idx], device=dev, dtype=torch.float64)
-    for m in nets:
-        m._cast_weights()
+    packed = [m._pack() for m in nets]
+    biases = [m.b for m in nets]
+    rule = (mu, sd, REGION_WEIGHT, TARGET_PERIOD, PERIOD_TOL, AMP_MIN, AMP_RAMP)
     n = P.shape[0]
     out = torch.empty(n, dtype=torch.float64, device=dev)
-    acc = torch.empty((batch, n_out), dtype=torch.float32, device=dev)
     for s in range(0, n, chunk):
         Pd = torch.as_tensor(np.ascontiguousarray(P[s:s + chunk], np.float64), device=dev)
+        if len(nets) <= MAX_NETS:
+            k.rank(Pd, idx_d, t_d, math.log(spread), packed, biases, n_out, *rule, out[s:s + Pd.shape[0]])
+            continue
         for b in range(0, Pd.shape[0], batch):
             rows = min(batch, Pd.shape[0] - b)
-            Bp = (rows + 127) // 128 * 128
-            Xb = nets[0]._buf("Xscore", (Bp, IN_PAD), torch.bfloat16)
+            Xb = torch.empty((rows, IN_PAD), dtype=torch.bfloat16, device=dev)
+            acc = torch.empty((rows, n_out), device=dev)
+            y = torch.empty((rows, n_out), device=dev)
             k.encode(Pd[b:b + rows], idx_d, t_d, math.log(spread), Xb)
+            x = Xb[:, :len(idx)].to(torch.float32)
             for i, m in enumerate(nets):
-                k.ensemble_accumulate(m.forward(Xb), rows, n_out, acc, i == 0)
-            k.score(acc[:rows], len(nets), mu, sd, REGION_WEIGHT, TARGET_PERIOD, PERIOD_TOL, AMP_MIN, AMP_RAMP,
-                    out[s + b:s + b + rows])
+                k.predict(x, packed[i], m.b, y)
+                k.ensemble_accumulate(y, rows, n_out, acc, i == 0)
+            k.score(acc, len(nets), *rule, out[s + b:s + b + rows])
     for m in nets:
         m.k.check()
     return out.cpu().numpy()

@@ -9,12 +9,14 @@ Every candidate it accepts is re-simulated by the FP64 engine, which alone
 decides acceptance.
 
 Network: in -> 3 x 256 (GELU) -> out, BF16 weights and activations on the
-GEMMs, FP32 accumulation, FP32 master weights with Adam.  Every matrix
-product of the forward and backward passes runs in the tcgen05 kernel of
-csrc/surrogate/umma_gemm.cuh; torch only allocates the buffers and orders
-the launches on one stream.
+products, FP32 accumulation, FP32 master weights with Adam.  Training,
+prediction and ranking run in the whole-network tcgen05 kernels of
+csrc/surrogate/chain.cu (``Kernels.gemm`` is the single product of
+umma_gemm_persistent.cuh); torch only allocates the buffers and orders the
+launches on one stream.
 """
 
+import concurrent.futures as cf
 import ctypes as C
 import os
 import subprocess
@@ -30,6 +32,7 @@ EPI_STORE, EPI_BIAS_GELU, EPI_BIAS = 0, 1, 2
 HIDDEN = 256
 IN_PAD = 64     # input features padded to the GEMM's K granularity
 OUT_PAD = 128   # outputs padded to one UMMA M tile for the weight gradient
+MAX_NETS = 64   # networks that one ranking launch takes
 
 
 def build(force=False):
@@ -41,18 +44,18 @@ def build(force=False):
     nvcc = os.environ.get("NVCC", "nvcc")
     base = [nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O3", "-lineinfo",
             "-I", os.path.join(os.path.dirname(HERE), "include")]
-    objs = []
-    cmds = []
-    for unit in ("mlp", "features"):
-        obj = os.path.join(LIB_DIR, "obj", unit + ".o")
-        objs.append(obj)
-        cmds.append(base + ["-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "-c",
-                            os.path.join(SRC, unit + ".cu"), "-o", obj])
-    cmds.append(base + ["-shared", "-o", LIB] + objs + ["-lcudart"])
-    for cmd in cmds:
+    units = ("mlp", "features", "chain")
+    objs = [os.path.join(LIB_DIR, "obj", unit + ".o") for unit in units]
+
+    def run(cmd):
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode:
             raise RuntimeError(r.stderr[-4000:])
+
+    with cf.ThreadPoolExecutor(len(units)) as ex:
+        list(ex.map(run, [base + ["-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "-c",
+                                  os.path.join(SRC, unit + ".cu"), "-o", obj] for unit, obj in zip(units, objs)]))
+    run(base + ["-shared", "-o", LIB] + objs + ["-lcudart"])
     return LIB
 
 
@@ -80,12 +83,25 @@ def lib():
         L.dense_features_ensemble_accumulate.argtypes = [vp, i, i, i, vp, i, vp]
         L.dense_features_score.argtypes = [vp, i, i, i, vp, vp, C.c_double, C.c_double, C.c_double, C.c_double,
                                            C.c_double, vp, vp]
+        L.dense_mlp_packed_bytes.restype = i64
+        L.dense_mlp_train_bytes.argtypes, L.dense_mlp_train_bytes.restype = [i, i], i64
+        L.dense_mlp_pack.argtypes = [vp, vp, i, vp]
+        L.dense_mlp_predict.argtypes = [vp, i, i, i, vp, vp, i, vp, vp, vp]
+        d = C.c_double
+        L.dense_mlp_rank.argtypes = [vp, i, i, vp, vp, i, d, i, vp, vp, i, vp, vp, d, d, d, d, d, vp, vp, vp]
+        L.dense_mlp_train_pass.argtypes = [vp, i, i, i, vp, vp, i, vp, i, vp, vp, vp, f, vp, vp, i64, vp, vp]
+        L.dense_mlp_train_finish.argtypes = [vp, i64, i, i] + [vp] * 11
         _lib = L
     return _lib
 
 
 def _p(t):
     return C.c_void_p(t.data_ptr()) if t is not None else None
+
+
+def _pp(ts):
+    """A host array of the tensors' device pointers (None: no array)."""
+    return None if ts is None else (C.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
 
 
 class Kernels:
@@ -194,6 +210,48 @@ class Kernels:
     def adam(self, w, g, m, v, lr, step, b1=0.9, b2=0.999, eps=1e-8):
         assert self.L.dense_mlp_adam(_p(w), _p(g), _p(m), _p(v), w.numel(), lr, b1, b2, eps, step, self._s()) == 0
 
+    def pack(self, W, packed, backward):
+        """The BF16 weights of one network in the order the whole-network
+        passes read them."""
+        assert self.L.dense_mlp_pack(_pp(W), _p(packed), int(backward), self._s()) == 0
+
+    def predict(self, X, packed, bias, out):
+        """out [rows][n_out] of the packed network for float32 rows X."""
+        n, n_in = X.shape
+        assert X.stride(1) == 1 or n_in == 1
+        assert self.L.dense_mlp_predict(_p(X), max(X.stride(0), n_in), n, n_in, _p(packed), _pp(bias), out.shape[1],
+                                        _p(out), _p(self.err), self._s()) == 0
+
+    def rank(self, P, idx, tmpl, log_spread, packed, biases, n_out, mu, sd, weight, period, tol, amp_min, ramp, out):
+        """Ranking scores of candidates P (float64 [n][params]) under the
+        ensemble of packed networks: encode, every network and score in one
+        launch."""
+        assert P.stride(1) == 1
+        mu = np.ascontiguousarray(mu, np.float32)
+        sd = np.ascontiguousarray(sd, np.float32)
+        assert self.L.dense_mlp_rank(_p(P), P.stride(0), P.shape[0], _p(idx), _p(tmpl), idx.shape[0],
+                                     float(log_spread), len(packed), _pp(packed), _pp([b for bs in biases for b in bs]),
+                                     n_out, mu.ctypes.data_as(C.c_void_p), sd.ctypes.data_as(C.c_void_p), weight,
+                                     period, tol, amp_min, ramp, _p(out), _p(self.err), self._s()) == 0
+
+    def train_pass(self, X, T, mask, idx, rows, packed, bias, inv_count, loss, work):
+        """One batch forward and back; inv_count a float, or a one-element
+        device tensor.  The gradients' parts stay in `work`."""
+        n, n_in = X.shape
+        dev_inv = inv_count if not isinstance(inv_count, float) else None
+        assert self.L.dense_mlp_train_pass(_p(X), n_in, n, n_in, _p(T), _p(mask), T.shape[1], _p(idx), rows,
+                                           _p(packed), _pp(bias), _p(dev_inv),
+                                           inv_count if dev_inv is None else 0.0, _p(loss), _p(work), work.numel(),
+                                           _p(self.err), self._s()) == 0
+
+    def train_finish(self, work, rows, n_out, dW=None, db=None, hyper=None, net=None):
+        """Gradients out of `work` into dW and db, and (with `hyper`) one
+        Adam step of `net`'s weights, packed for the next pass."""
+        state = (net.W, net.b, net.mW, net.vW, net.mb, net.vb) if hyper is not None else (None,) * 6
+        assert self.L.dense_mlp_train_finish(_p(work), work.numel(), rows, n_out, _pp(dW), _pp(db), _p(hyper),
+                                             *[_pp(t) for t in state], _p(net._packed if net else None),
+                                             self._s()) == 0
+
     def check(self):
         self.torch.cuda.synchronize(self.dev)
         e = int(self.err.item())
@@ -204,10 +262,10 @@ class Kernels:
 class MLP:
     """in -> 3 x 256 GELU -> out on the tensor-core kernels.
 
-    Weights are kept as FP32 masters [out][in] with Adam moments; every step
-    casts them to BF16 (and transposed BF16 copies for the input-gradient
-    products).  Inputs are padded to IN_PAD features and outputs to OUT_PAD
-    rows (the padding weights stay zero: their gradients are zero).
+    Weights are kept as FP32 masters [out][in] with Adam moments; the passes
+    read BF16 copies packed in their own order.  Inputs are padded to IN_PAD
+    features and outputs to OUT_PAD rows (the padding weights stay zero:
+    their gradients are zero).
     """
 
     def __init__(self, n_in, n_out, seed=0, device=0, lr=1e-3, group=None):
@@ -247,112 +305,71 @@ class MLP:
             self._bufs[name] = t
         return t
 
-    def _cast_weights(self):
-        bf = self.torch.bfloat16
-        self.Wb = [self._buf("Wb%d" % i, w.shape, bf) for i, w in enumerate(self.W)]
-        self.WTb = [self._buf("WTb%d" % i, (w.shape[1], w.shape[0]), bf) for i, w in enumerate(self.W)]
-        for i, w in enumerate(self.W):
-            self.k.cast(w, self.Wb[i])
-            if i > 0:
-                self.k.cast(w, self.WTb[i], transpose=True)
+    @property
+    def _packed(self):
+        return self._buf("packed", (int(self.k.L.dense_mlp_packed_bytes()),), self.torch.uint8)
 
-    def _input(self, X):
-        """[B][n_in] float -> padded BF16 [Bp][IN_PAD], Bp a multiple of 128."""
-        B = X.shape[0]
-        Bp = (B + 127) // 128 * 128
-        Xb = self._buf("Xb", (Bp, IN_PAD), self.torch.bfloat16)
-        Xb.zero_()
-        Xb[:B, :self.n_in] = self.torch.as_tensor(X, device=self.dev, dtype=self.torch.float32).to(self.torch.bfloat16)
-        return Xb, Bp
+    def _pack(self, backward=False):
+        self.k.pack(self.W, self._packed, backward)
+        return self._packed
 
-    def forward(self, Xb):
-        Bp = Xb.shape[0]
-        bf = self.torch.bfloat16
-        self.Z = [self._buf("Z%d" % i, (Bp, HIDDEN)) for i in range(3)]
-        self.H = [Xb] + [self._buf("H%d" % i, (Bp, HIDDEN), bf) for i in range(1, 4)]
-        for i in range(3):
-            self.k.gemm(self.H[i], self.Wb[i], self.Z[i], EPI_BIAS_GELU, self.b[i], self.H[i + 1])
-        Y = self._buf("Y", (Bp, OUT_PAD))
-        self.k.gemm(self.H[3], self.Wb[3], Y, EPI_BIAS, self.b[3])
-        return Y
+    def _rows(self, X):
+        """Float32 CUDA rows [B][n_in] of X, each value rounded as it would
+        be to BF16 (once)."""
+        torch = self.torch
+        X = X.detach()
+        if X.dtype != torch.float32:
+            X = X.to(torch.bfloat16).to(torch.float32)
+        X = X.to(self.dev).expand(X.shape[0], self.n_in)
+        return X if X.stride(1) == 1 and X.stride(0) >= self.n_in else X.contiguous()
 
     def predict_device(self, X, batch=65536):
         """Outputs [B][n_out] as a CUDA float32 tensor, for inputs already
-        on the GPU (a float tensor [B][n_in]); nothing crosses to the host."""
-        torch = self.torch
-        self._cast_weights()
-        out = []
-        for s in range(0, X.shape[0], batch):
-            x = X[s:s + batch]
-            B = x.shape[0]
-            Bp = (B + 127) // 128 * 128
-            Xb = self._buf("Xb", (Bp, IN_PAD), torch.bfloat16)
-            Xb.zero_()
-            Xb[:B, :self.n_in] = x.to(torch.bfloat16)
-            Y = self.forward(Xb)
-            out.append(Y[:B, :self.n_out].clone())
+        on the GPU (a float tensor [B][n_in]); nothing crosses to the host.
+        One launch carries every row through the whole network (`batch` is
+        kept for callers that pass it)."""
+        out = self.torch.empty((X.shape[0], self.n_out), device=self.dev)
+        self.k.predict(self._rows(X), self._pack(), self.b, out)
         self.k.check()
-        return torch.cat(out) if out else torch.zeros((0, self.n_out), device=self.dev)
+        return out
 
     def predict(self, X, batch=65536):
         """Outputs [B][n_out] (float32, on the host)."""
-        self._cast_weights()
+        torch = self.torch
+        packed = self._pack()
         out = []
         for s in range(0, X.shape[0], batch):
-            Xb, _ = self._input(X[s:s + batch])
-            Y = self.forward(Xb)
-            out.append(Y[:min(batch, X.shape[0] - s), :self.n_out].float().cpu().numpy())
+            x = torch.as_tensor(X[s:s + batch], device=self.dev, dtype=torch.float32)
+            y = torch.empty((x.shape[0], self.n_out), device=self.dev)
+            self.k.predict(self._rows(x), packed, self.b, y)
+            out.append(y.cpu().numpy())
         self.k.check()
         return np.concatenate(out) if out else np.zeros((0, self.n_out), np.float32)
 
+    def _work(self, rows):
+        return self._buf("work", (int(self.k.L.dense_mlp_train_bytes(rows, self.n_out)),), self.torch.uint8)
+
+    def _grads(self):
+        return ([self._buf("dW%d" % i, w.shape) for i, w in enumerate(self.W)],
+                [self._buf("db%d" % i, b.shape) for i, b in enumerate(self.b)])
+
     def gradients(self, X, T, mask):
-        """Loss and gradients (dW, db lists) of one batch; Bp rows, padding masked."""
+        """Loss and gradients (dW, db lists) of one batch."""
         torch = self.torch
-        bf = torch.bfloat16
-        self._cast_weights()
-        Xb, Bp = self._input(X)
         B = X.shape[0]
-        Tt = torch.zeros((Bp, self.n_out), device=self.dev)
-        Mt = torch.zeros((Bp, self.n_out), device=self.dev)
-        Tt[:B] = torch.as_tensor(np.nan_to_num(T), device=self.dev, dtype=torch.float32)
-        Mt[:B] = torch.as_tensor(mask, device=self.dev, dtype=torch.float32)
-        Y = self.forward(Xb)
+        f32 = dict(device=self.dev, dtype=torch.float32)
+        x = torch.as_tensor(X, **f32).expand(B, self.n_in).contiguous()
+        t = torch.as_tensor(np.nan_to_num(T), **f32).expand(B, self.n_out).contiguous()
+        m = torch.as_tensor(mask, **f32).expand(B, self.n_out).contiguous()
+        count = float(m.sum().item() if torch.is_tensor(mask) else
+                      np.broadcast_to(np.asarray(mask, np.float32), (B, self.n_out)).sum(dtype=np.float64))
         loss = torch.zeros(1, device=self.dev)
-        dY = self._buf("dY", (Bp, OUT_PAD))
-        dYb = self._buf("dYb", (Bp, OUT_PAD), bf)
-        self.k.mse(Y, Tt, Mt, dY, dYb, loss)
-        dW, db = self._backward(dY, dYb, Bp)
+        dW, db = self._grads()
+        work = self._work(B)
+        self.k.train_pass(x, t, m, None, B, self._pack(backward=True), self.b, 1.0 / max(1.0, count), loss, work)
+        self.k.train_finish(work, B, self.n_out, dW, db)
         self.k.check()
         return float(loss.item()), dW, db
-
-    def _backward(self, dY, dYb, Bp):
-        """Weight and bias gradients from the output gradient dY (FP32 and
-        BF16 copies) of the last forward pass over Bp rows."""
-        bf = self.torch.bfloat16
-        dW = [None] * 4
-        db = [None] * 4
-        dZ, dZb = dY, dYb
-        for i in (3, 2, 1, 0):
-            rows = self.W[i].shape[0]
-            # weight gradient: dW_i = dZ^T H_i  (M = out rows, N = in, K = batch)
-            dZT = self._buf("dZT%d" % i, (rows, Bp), bf)
-            HT = self._buf("HT%d" % i, (self.W[i].shape[1], Bp), bf)
-            self.k.transpose(dZb, dZT)
-            self.k.transpose(self.H[i], HT)
-            dW[i] = self._buf("dW%d" % i, self.W[i].shape)
-            self.k.gemm(dZT, HT, dW[i])
-            db[i] = self._buf("db%d" % i, (rows,))
-            self.k.colsum(dZ, db[i])
-            if i == 0:
-                break
-            # input gradient: dH_i = dZ W_i, then dZ_{i-1} = dH_i * GELU'(Z_{i-1})
-            dH = self._buf("dH%d" % i, (Bp, HIDDEN))
-            self.k.gemm(dZb, self.WTb[i], dH)
-            ndZ = self._buf("dZ%d" % (i - 1), (Bp, HIDDEN))
-            ndZb = self._buf("dZb%d" % (i - 1), (Bp, HIDDEN), bf)
-            self.k.gelu_backward(dH, self.Z[i - 1], ndZ, ndZb)
-            dZ, dZb = ndZ, ndZb
-        return dW, db
 
     def _train_graphs(self, data, batch, steps):
         """CUDA graphs of training on the device-resident training set
@@ -360,51 +377,51 @@ class MLP:
         Per epoch the host writes the epoch's row indices ("idx", steps x
         batch) and per-step scalars ("hyper", steps x {lr, b1, b2, eps,
         1 - b1^t, 1 - b2^t, 1 / count}) into static device buffers.  One
-        process: one graph replays the whole epoch (per step: batch gather,
-        weight casts, forward, loss, backward, Adam).  Data-parallel: per
+        process: one graph replays the whole epoch, three launches per step
+        (the batch forward and back, the weight gradients, Adam and the
+        weights' next layout).  Data-parallel: per
         step a gradient graph and an update graph, with the gradient
         all-reduce between them.  The graphs hold the addresses of this
         object's work buffers: they serve one fit call only (no other pass
         may resize a buffer meanwhile)."""
         torch = self.torch
-        Bp = (batch + 127) // 128 * 128
-        bf = torch.bfloat16
-        g = {"Bp": Bp}
+        g = {}
         g["idx"] = torch.zeros(steps * batch, dtype=torch.int32, device=self.dev)
         g["hyper"] = torch.zeros((steps, 8), device=self.dev)
         g["loss"] = torch.zeros(1, device=self.dev)
         Xd, Td, Md = data
+        work = self._work(batch)
+        packed = self._packed
+        dW, db = g["dW"], g["db"] = self._grads()
+
+        def pass_(j):
+            self.k.train_pass(Xd, Td, Md, g["idx"][j * batch:(j + 1) * batch], batch, packed, self.b,
+                              g["hyper"][j, 6:7], g["loss"], work)
 
         def grads(j):
-            self._cast_weights()
-            Xb = self._buf("Xb", (Bp, IN_PAD), bf)
-            Tb = self._buf("Tb", (Bp, self.n_out))
-            Mb = self._buf("Mb", (Bp, self.n_out))
-            self.k.gather(Xd, Td, Md, g["idx"][j * batch:(j + 1) * batch], Xb, Tb, Mb)
-            Y = self.forward(Xb)
-            dY = self._buf("dY", (Bp, OUT_PAD))
-            dYb = self._buf("dYb", (Bp, OUT_PAD), bf)
-            self.k.mse_dev(Y, Tb, Mb, g["hyper"][j, 6:7], dY, dYb, g["loss"])
-            g["dW"], g["db"] = self._backward(dY, dYb, Bp)
+            self._pack(backward=True)
+            pass_(j)
+            self.k.train_finish(work, batch, self.n_out, dW, db)
 
         def update(j):
             hyper = g["hyper"][j]
             for i in range(4):
-                self.k.adam_dev(self.W[i], g["dW"][i], self.mW[i], self.vW[i], hyper)
-                self.k.adam_dev(self.b[i], g["db"][i], self.mb[i], self.vb[i], hyper)
+                self.k.adam_dev(self.W[i], dW[i], self.mW[i], self.vW[i], hyper)
+                self.k.adam_dev(self.b[i], db[i], self.mb[i], self.vb[i], hyper)
 
         side = torch.cuda.Stream(self.dev)
         side.wait_stream(torch.cuda.current_stream(self.dev))
         with torch.cuda.stream(side):
-            grads(0)  # allocates every buffer before capture; changes no weight
+            grads(0)  # a first launch of each kernel before capture; changes no weight
         torch.cuda.current_stream(self.dev).wait_stream(side)
         torch.cuda.synchronize(self.dev)
         if self.group is None:
             g["epoch"] = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g["epoch"]):
+                self._pack(backward=True)
                 for j in range(steps):
-                    grads(j)
-                    update(j)
+                    pass_(j)
+                    self.k.train_finish(work, batch, self.n_out, hyper=g["hyper"][j], net=self)
         else:
             g["grads"], g["update"] = [], []
             for j in range(steps):
