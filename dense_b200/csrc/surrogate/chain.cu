@@ -25,7 +25,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
-#include "dense_b200_surrogate.h"
+#include "dense_b200_network.h"
 
 #include <atomic>
 #include <cmath>

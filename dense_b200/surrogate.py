@@ -36,14 +36,15 @@ MAX_NETS = 64   # networks that one ranking launch takes
 
 
 def build(force=False):
-    srcs = [os.path.join(SRC, f) for f in os.listdir(SRC)] + [os.path.join(os.path.dirname(HERE), "include",
-                                                                            "dense_b200_surrogate.h")]
+    include = os.path.join(os.path.dirname(HERE), "include")
+    srcs = [os.path.join(SRC, f) for f in os.listdir(SRC)] + [os.path.join(include, f) for f in
+                                                              ("dense_b200_surrogate.h", "dense_b200_network.h")]
     if not force and os.path.exists(LIB) and all(os.path.getmtime(s) <= os.path.getmtime(LIB) for s in srcs):
         return LIB
     os.makedirs(os.path.join(LIB_DIR, "obj"), exist_ok=True)
     nvcc = os.environ.get("NVCC", "nvcc")
     base = [nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O3", "-lineinfo",
-            "-I", os.path.join(os.path.dirname(HERE), "include")]
+            "-I", include]
     units = ("mlp", "features", "chain")
     objs = [os.path.join(LIB_DIR, "obj", unit + ".o") for unit in units]
 
