@@ -657,13 +657,17 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
     }
     lvl_cells_all.insert(lvl_cells_all.end(), plan.lvl_cells.begin(), plan.lvl_cells.end());
     if (plan.wave) {
-      // cell records in level order: {cell, neighbour count, ids (ascending), 0...}
+      // cell records in level order: {cell, neighbour count and (high byte)
+      // how many of them have lower ids, ids (ascending), 0...}
       d.rec_base = static_cast<int64_t>(rec_all.size() / 8);
       for (int i = 0; i < n; ++i) {
         const int c = plan.lvl_cells[i];
         const int k0 = in.nbr_offsets[c], cnt = in.nbr_offsets[c + 1] - k0;
         uint16_t r[8] = {static_cast<uint16_t>(c), static_cast<uint16_t>(cnt), 0, 0, 0, 0, 0, 0};
-        for (int e = 0; e < cnt; ++e) r[2 + e] = static_cast<uint16_t>(in.nbr_ids[k0 + e]);
+        for (int e = 0; e < cnt; ++e) {
+          r[2 + e] = static_cast<uint16_t>(in.nbr_ids[k0 + e]);
+          if (in.nbr_ids[k0 + e] < c) r[1] += 256;
+        }
         rec_all.insert(rec_all.end(), r, r + 8);
       }
     }

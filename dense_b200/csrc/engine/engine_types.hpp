@@ -82,8 +82,8 @@ struct SetDesc {
   int n_levels;          // memory kernel: cell-dependency levels per step
   int ordered;           // neighbour reads of the row written in the same step (DENSE's cell order)
   // wave kernel (ordered sets): rows indexed modulo D (not a power of two),
-  // cells as 16-byte records {cell, neighbour count, up to 6 neighbour ids}
-  // in level order
+  // cells as 16-byte records {cell, neighbour count | lower-numbered
+  // neighbours << 8, up to 6 neighbour ids} in level order
   int wave;
   int smem_off[kNS];     // byte offset of the species' rows in shared memory, -1: global
   int lvl_smem_off;      // byte offset of the 16-bit level offsets in shared memory
