@@ -1407,8 +1407,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_wave_kernel(c
   const int delta = sd.wave_delta;
   const int gsz = blk / fronts;
   const int grp = tid / gsz, gtid = tid % gsz;
+  // without analyses nothing happens between chunks, and the wavefronts run
+  // through many of them instead of draining after each (10 steps a chunk,
+  // 141 levels 48 apart: 480 intervals a chunk instead of 573)
+  const int64_t intervals = max(static_cast<int64_t>(sd.steps_per_chunk) * max(1, delta), int64_t(1));
+  const int together = a.n_analyses > 0 ? 1 : static_cast<int>(max((int64_t(1) << 26) / intervals, int64_t(1)));
 
-  for (; chunk < chunk_end; ++chunk) {
+  for (int chunks = 1; chunk < chunk_end; chunk += chunks) {
+    chunks = min(together, chunk_end - chunk);
     if (a.n_analyses > 0) {
       for (int i = tid; i < kNS; i += blk) {
         const int row = a.val_slot[i];
@@ -1433,10 +1439,13 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_wave_kernel(c
     // k = g (mod fronts); a barrier closes each interval.  A group meets its
     // steps in order, fronts * delta intervals apart, so it counts its level
     // up instead of dividing tau (a warp's instructions are the interval's
-    // length: with the divisions, the select of each neighbour's row by its
-    // id and the proven division 380 of them, now 190; 48 x 48 grids, 200
-    // steps: 9.5 -> 5.6 ms)
-    const int S_chunk = sd.steps_per_chunk;
+    // length, 3.9 cycles each: with the divisions, the select of each
+    // neighbour's row by its id and the proven division some 380 of them, now
+    // 222; 200 grids of 8 x 8 to 48 x 48, 200 steps: 9.07 -> 4.92 ms.
+    // Fetching the next level's record and state before the barrier cost more
+    // instructions than the latency it hid, 5.4 ms; 32-bit row offsets in
+    // place of pointers 5.1 ms.)
+    const int S_chunk = sd.steps_per_chunk * chunks;
     const int n_intervals = S_chunk > 0 ? (S_chunk - 1) * delta + n_levels : 0;
     const int period = fronts * delta;
     int l = -grp * delta - 1;               // this group's level in interval tau (negative: not begun)
@@ -1508,7 +1517,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_wave_kernel(c
       __syncthreads();
     }
     step += S_chunk;
-    age += a.interval;
+    for (int i = 0; i < chunks; ++i) age += a.interval;
   }
 
   // lag-0 state to the state block (what read_state returns), shared rows
