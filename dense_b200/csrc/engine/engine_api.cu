@@ -70,6 +70,7 @@ struct SetPlan {
   bool use_mem = false;         // run by the memory-state kernel (or the wave kernel)
   bool wave = false;            // an ordered set run by the wave kernel
   int mem_block = 256;          // its CTA size
+  int ranks = 0;                // > 0: run by the register kernel over a cluster of so many CTAs
   std::vector<int> lvl_off;     // memory kernel: level offsets into lvl_cells
   std::vector<int> lvl_cells;   // memory kernel: cells in level order
 };
@@ -214,8 +215,8 @@ struct dense_engine {
   int n_reg = 0, n_mem = 0;  // sets run by the register / memory kernels (d_lists: reg then mem)
   // memory- and wave-kernel sets in launch groups of one kernel, CTA size
   // and dynamic shared memory: (kernel: 0 memory, 1 wave, 2 wave with
-  // everything shared; threads; shared bytes; first index in the mem list;
-  // count)
+  // everything shared, 3 register kernel over clusters; threads; shared
+  // bytes, or CTAs per cluster; first index in the mem list; count)
   std::vector<std::array<int, 5>> mem_groups;
   std::map<int, cudaGraphExec_t> graphs;
   // the kernel launches of one run (register kernel, one per memory- or
@@ -393,6 +394,11 @@ int plan_set(const dense_set_desc& in, double dt, int elem_bytes, SetPlan& plan,
     for (int c = 0; c < n; ++c)
       if (in.nbr_offsets[c + 1] - in.nbr_offsets[c] > kWaveMaxNbrs) plan.wave = false;
   }
+  // tissues too large for one CTA run in the register kernel, spread over a
+  // cluster, unless a hint asks for the memory kernel; their rings keep the
+  // memory kernel's layout, so either can go on from the other's run state
+  const int ranks = (n + kStepThreads - 1) / kStepThreads;
+  if (!ordered && !force_mem && n > kStepThreads && in.mem_block == 0 && ranks <= kMaxCluster) plan.ranks = ranks;
   // memory-kernel CTA size: the hint, else the widest level in warps (32..256)
   int widest = 0;
   for (size_t l = 0; l + 1 < plan.lvl_off.size(); ++l) widest = std::max(widest, plan.lvl_off[l + 1] - plan.lvl_off[l]);
@@ -415,6 +421,7 @@ int plan_set(const dense_set_desc& in, double dt, int elem_bytes, SetPlan& plan,
   stage();
   // the register kernel forms ring offsets in 32 bits and packs lags in 26;
   // larger rings (no model's delays come near) go to the memory kernel
+  if (off > kMaxRegisterRing) plan.ranks = 0;
   if (!plan.use_mem && off > kMaxRegisterRing) {
     plan.use_mem = true;
     stage();
@@ -598,6 +605,14 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
   std::vector<uint16_t> rec_all;  // wave-kernel cell records, 8 x 16 bits each
   e->sets.resize(num_sets);
   e->init_status.resize(num_sets);
+  bool sampled[NUM_SPECIES] = {};
+  size_t sample_bytes = 0;  // shared memory of a cluster CTA's sampled state
+  for (const AnalysisDesc& A : e->analyses)
+    for (int i = 0; i < A.nsp; ++i)
+      if (!sampled[A.sp[i]]) {
+        sampled[A.sp[i]] = true;
+        sample_bytes += sizeof(double) * kStepThreads;
+      }
   std::vector<double> cp;
   for (int s = 0; s < num_sets; ++s) {
     const dense_set_desc& in = in_sets[s];
@@ -612,6 +627,7 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
     SetPlan plan;
     int rc = plan_set(in, dt, run->precision == DENSE_FP64 ? 8 : 4, plan, cp);
     if (rc != DENSE_OK) return fail(rc, where + g_error);
+    if (sample_bytes > kClusterSmem) plan.ranks = 0;
     SetDesc& d = plan.d;
     const double chunks = in.duration / interval;  // run_simulation.hpp:127
     if (!(chunks < 2147483647.0)) return fail(DENSE_ERR_INVALID, where + "too many chunks");
@@ -647,7 +663,11 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
       mem_smem_of.push_back(plan.wave ? wave_smem_bucket(d.smem_bytes) : -1);
       bool all_shared = plan.wave && d.topo_off >= 0;
       for (int sp = 0; sp < NUM_SPECIES; ++sp) all_shared = all_shared && d.smem_off[sp] >= 0;
-      mem_kind_of.push_back(plan.wave ? (all_shared ? 2 : 1) : 0);
+      mem_kind_of.push_back(plan.wave ? (all_shared ? 2 : 1) : (plan.ranks > 0 ? 3 : 0));
+      if (plan.ranks > 0) {
+        mem_block_of.back() = ((n + plan.ranks - 1) / plan.ranks + 31) / 32 * 32;  // cells per CTA
+        mem_smem_of.back() = plan.ranks;
+      }
       d.lvl_base = static_cast<int64_t>(lvl_off_all.size());
       lvl_off_all.insert(lvl_off_all.end(), plan.lvl_off.begin(), plan.lvl_off.end());
     } else {
@@ -718,8 +738,8 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
     std::stable_sort(reg_list.begin(), reg_list.end(), by_cost);
     // memory- and wave-kernel sets: grouped by kernel, CTA size and shared
     // memory bucket (-1: memory kernel), longest first in a group
-    // key: (kernel: 0 memory, 1 wave, 2 wave with everything shared; shared
-    // memory bucket; CTA size)
+    // key: (kernel, as in mem_groups; shared memory bucket or CTAs per
+    // cluster; CTA size)
     std::vector<std::array<int, 3>> key_of(num_sets, {0, 0, 0});
     for (size_t k = 0; k < mem_list.size(); ++k)
       key_of[mem_list[k]] = {mem_kind_of[k], std::max(0, mem_smem_of[k]), mem_block_of[k]};
@@ -750,8 +770,9 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
       double m = 0;
       for (int j = g[3]; j < g[3] + g[4]; ++j) {
         const SetDesc& d = e->sets[mem_list[j]];
-        const double per_step = g[0] ? d.wave_delta : d.n_levels * std::ceil(static_cast<double>(d.n_cells) /
-                                                                            (d.n_levels * g[1]));
+        const double per_step = g[0] == 3 ? 1
+                                : g[0]    ? d.wave_delta
+                                          : d.n_levels * std::ceil(static_cast<double>(d.n_cells) / (d.n_levels * g[1]));
         m = std::max(m, static_cast<double>(d.n_chunks) * d.steps_per_chunk * per_step);
       }
       est.push_back({m, k++});
@@ -884,7 +905,10 @@ static cudaError_t launch_all(dense_engine* e, const StepArgs& a, cudaStream_t s
   }
   for (const auto& g : e->mem_groups) {
     if ((r = stream_for(st)) != cudaSuccess) return r;
-    if (g[0])
+    if (g[0] == 3)
+      r = e->precision == DENSE_FP64 ? launch_step_cluster_fp64(a, mem + g[3], g[4], g[1], g[2], st)
+                                     : launch_step_cluster_fp32(a, mem + g[3], g[4], g[1], g[2], st);
+    else if (g[0])
       r = e->precision == DENSE_FP64 ? launch_step_wave_fp64(a, mem + g[3], g[4], g[1], g[2], g[0] == 2, st)
                                      : launch_step_wave_fp32(a, mem + g[3], g[4], g[1], g[2], g[0] == 2, st);
     else

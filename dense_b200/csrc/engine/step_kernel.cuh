@@ -23,6 +23,7 @@
 // the model's reaction_deltas.hpp and model_impl.hpp first.
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "count_div.cuh"
@@ -228,7 +229,10 @@ enum ReadMode : int {
 //    that their L2 latencies overlap;
 //  * flagged reads leave no branch in either pass: they only mark the step,
 //    and a marked step runs the checked pass instead.
-template <typename T, bool kTable, int kMode>
+//
+// kFar: the set's cells are spread over a cluster, so neighbours' rows are
+// written by other SMs and read past the L1.
+template <typename T, bool kTable, int kMode, bool kFar>
 struct RegContext {
   const T* cur;            // this cell's lag-0 state [NS] (registers)
   const T* prm;            // parameters: shared row (pstride 1) or this cell's column (pstride n)
@@ -253,19 +257,21 @@ struct RegContext {
     return ((step - lag) & r.x) * n_cells + r.y;
   }
 
+  static __device__ __forceinline__ T far(const T* p) { return kFar ? __ldcg(p) : *p; }
+
   // DENSE's average over the neighbours: ascending ids, sum / count, NaN -> 0.
   __device__ __forceinline__ T average(const T* row) const {
     T sum = T(0);
     if (nnbr <= kSmallCount) {
       // absent neighbours' ids are 0: their loads stay in the row
-      const T v[6] = {row[nb01 & 0xFFFFu], row[nb01 >> 16], row[nb23 & 0xFFFFu],
-                      row[nb23 >> 16],     row[nb45 & 0xFFFFu], row[nb45 >> 16]};
+      const T v[6] = {far(row + (nb01 & 0xFFFFu)), far(row + (nb01 >> 16)), far(row + (nb23 & 0xFFFFu)),
+                      far(row + (nb23 >> 16)),     far(row + (nb45 & 0xFFFFu)), far(row + (nb45 >> 16))};
 #pragma unroll
       for (int e = 0; e < 6; ++e)
         if (e < nnbr) sum += v[e];
       if (small_count_operand(sum)) return div_by_small_count(sum, static_cast<T>(nnbr), rc);
     } else {
-      for (int e = 0; e < nnbr; ++e) sum += row[nbr[e]];
+      for (int e = 0; e < nnbr; ++e) sum += far(row + nbr[e]);
     }
     const T avg = sum / static_cast<T>(nnbr);
     return isnan(avg) ? T(0) : avg;
@@ -344,8 +350,8 @@ struct RegContext {
 
   // the same context for another pass
   template <int kOther>
-  __device__ __forceinline__ RegContext<T, kTable, kOther> as() const {
-    return RegContext<T, kTable, kOther>{cur, prm, pstride, own_at, nbr_at, S,    rows, ring, step,
+  __device__ __forceinline__ RegContext<T, kTable, kOther, kFar> as() const {
+    return RegContext<T, kTable, kOther, kFar>{cur, prm, pstride, own_at, nbr_at, S,    rows, ring, step,
                                          nbr, nnbr, nb01,   nb23,   nb45,   rc,   n_cells, cell, err, f};
   }
 };
@@ -624,10 +630,26 @@ __device__ __forceinline__ void osc_cell_finalize(double* st, const AnalysisDesc
 // Where the analyses read the sampled state: the shared staging buffer of
 // the register kernel, or the lag-0 rows of the rings in the memory kernel.
 struct SmemVals {
-  const double* base;
+  const double* base;  // of the CTA's first cell
   int blk;
-  __device__ __forceinline__ double operator()(int slot, int cell) const { return base[slot * blk + cell]; }
+  int first;
+  __device__ __forceinline__ double operator()(int slot, int cell) const { return base[slot * blk + cell - first]; }
 };
+
+// The same over a cluster whose CTAs hold `blk` cells each.
+struct ClusterVals {
+  double* base;
+  int blk;
+  __device__ __forceinline__ double operator()(int slot, int cell) const {
+    const int rank = cell / blk;
+    return cooperative_groups::this_cluster().map_shared_rank(base, rank)[slot * blk + cell - rank * blk];
+  }
+};
+
+// All threads of the cluster; what they wrote before is visible after.
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
 
 template <typename T>
 struct RingVals {
@@ -643,31 +665,34 @@ struct RingVals {
 
 // One analysis sample of a set at `age` (measurement/base.ipp:4-9): every
 // analysis records the time; those whose window contains it update, over
-// the cells c0, c0 + stride, ... this thread handles.  Returns whether a
-// concentration check failed for one of them.
-template <typename Vals>
-__device__ __forceinline__ bool analyses_sample(const StepArgs& a, double* anl, const Vals& vals, int tid, int c0,
-                                                int stride, int n, double age, const double* samples) {
+// the cells c0, c0 + stride, ... this thread handles.  `fold` reads any cell
+// of the set; with `lead` this CTA does what is done once per set (tid 0,
+// and the whole-range folds of warp 0).  Returns whether a concentration
+// check failed for one of the thread's cells.
+template <typename Vals, typename Fold>
+__device__ __forceinline__ bool analyses_sample(const StepArgs& a, double* anl, const Vals& vals, const Fold& fold,
+                                                bool lead, int tid, int c0, int stride, int n, double age,
+                                                const double* samples) {
   bool bad = false;
   for (int ai = 0; ai < a.n_analyses; ++ai) {
     const AnalysisDesc& A = a.analyses[ai];
     double* st = anl + A.off;
     const bool in_range = !(age < A.t0 || age >= A.t1);
     if (A.kind == kBasic) {
-      if (tid == 0) st[3 * A.nsp + 1] = age;
+      if (lead && tid == 0) st[3 * A.nsp + 1] = age;
       if (!in_range) continue;
       for (int c = c0; c < n; c += stride) basic_cell_update(st, A, vals, c);
-      if (tid < 32) basic_range_fold(st, A, vals, tid);
-      if (tid == 0) st[3 * A.nsp] += 1.0;
+      if (lead && tid < 32) basic_range_fold(st, A, fold, tid);
+      if (lead && tid == 0) st[3 * A.nsp] += 1.0;
     } else if (A.kind == kOscillation) {
-      if (tid == 0) st[1] = age;
+      if (lead && tid == 0) st[1] = age;
       if (!in_range) continue;
       for (int c = c0; c < n; c += stride) osc_cell_update(st, A, vals, c, samples[ai]);
-      if (tid == 0) st[0] = samples[ai] + 1.0;
+      if (lead && tid == 0) st[0] = samples[ai] + 1.0;
     } else if (A.kind == kTrajectory) {
       // csvw_sim::update (io/csvw_sim.ipp:17-91): every observed species
       // of every analysed cell at every sample
-      if (tid == 0) st[1] = age;
+      if (lead && tid == 0) st[1] = age;
       if (!in_range) continue;
       // the count as it was before this sample: thread 0 advances st[0] below
       // while other warps may still be here
@@ -679,11 +704,11 @@ __device__ __forceinline__ bool analyses_sample(const StepArgs& a, double* anl, 
           if (c < A.cmin || c >= A.cmax) continue;
           for (int i = 0; i < A.nsp; ++i) vals_k[static_cast<size_t>(i) * m + (c - A.cmin)] = vals(A.slot[i], c);
         }
-        if (tid == 0) st[2 + k] = age;
+        if (lead && tid == 0) st[2 + k] = age;
       }
-      if (tid == 0) st[0] = static_cast<double>(k + 1);
+      if (lead && tid == 0) st[0] = static_cast<double>(k + 1);
     } else if (A.kind == kConcCheck) {
-      if (tid == 0) st[0] = age;
+      if (lead && tid == 0) st[0] = age;
       if (!in_range) continue;
       for (int c = c0; c < n; c += stride) {
         if (c < A.cmin || c >= A.cmax) continue;
@@ -703,7 +728,16 @@ __device__ __forceinline__ bool analyses_sample(const StepArgs& a, double* anl, 
 // of up to 224 cells (128 registers: the fourteen warps put four on the
 // busiest of the SM's four sub-partitions, whose register file holds
 // 16384), 256 threads with one CTA per SM above that.
-template <typename T, bool kKahan, int kThreads, int kMinBlocks, bool kUniform>
+//
+// kCluster: a set's cells are spread over the CTAs of a cluster (blockDim
+// cells each), which meet at a cluster barrier after each step; for tissues
+// of more than 256 cells.  The memory kernel, which walks such a set with one
+// CTA and keeps the state in the rings, took 4.82 ms for 96 sets x 733 cells
+// x 200 steps; three CTAs a set take 2.84 ms, and 93 sets, all the clusters
+// of three that the GPU holds at once, 1.02 ms (5.1 us a step, of which the
+// cluster barrier and the release of the rows written before it are a
+// quarter).
+template <typename T, bool kKahan, int kThreads, int kMinBlocks, bool kUniform, bool kCluster>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const StepArgs a, const int* set_list) {
   // dynamic shared memory: sampled state [n_vals][blockDim] (doubles, only
   // with analyses) | the set's neighbour ids
@@ -724,12 +758,16 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
   __shared__ unsigned short s_live[kEntries > 0 ? kEntries : 1];
   __shared__ int s_n_live;
 
-  const int set = set_list[blockIdx.x];
+  namespace cg = cooperative_groups;
+  const int ranks = kCluster ? static_cast<int>(cg::this_cluster().num_blocks()) : 1;
+  const int rank = kCluster ? static_cast<int>(cg::this_cluster().block_rank()) : 0;
+  const int set = set_list[kCluster ? blockIdx.x / ranks : blockIdx.x];
   const SetDesc& sd = a.sets[set];
   const int n = sd.n_cells;
   const int blk = blockDim.x;
   const int c = threadIdx.x;
-  const bool active = c < n;
+  const int first = rank * blk;  // this CTA's cells: first, first + 1, ...
+  const bool active = first + c < n;
 
   const SetProgress pg = a.prog[set];
   if ((pg.status & (kSetDropped | kSetNotRunnable)) || pg.finalized) return;
@@ -751,7 +789,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
   if (c < a.n_analyses) s_samples[c] = anl[a.analyses[c].off];
   __syncthreads();
 
-  const int cell = active ? c : 0;
+  const int cell = active ? first + c : 0;
   // parameters: the shared row of the set, or this cell's column of the
   // set's [NP][n] block (read through L1)
   const T* prm = pstride == 0 ? s_prm : P + cell;
@@ -815,7 +853,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
   uint32_t nb[6];
 #pragma unroll
   for (int e = 0; e < 6; ++e) nb[e] = e < nnbr ? static_cast<uint32_t>(nbr[e]) : 0u;
-  if (a.csr_in_smem) {
+  if (!kCluster && a.csr_in_smem) {
     // the set's neighbour ids, [edges], in shared memory
     int* s_csr = reinterpret_cast<int*>(s_dyn + (a.n_analyses > 0 ? a.n_vals * blk : 0));
     const int e0 = nbr_off[0], ne = nbr_off[n] - e0;
@@ -828,7 +866,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
   T* ring = static_cast<T*>(a.ring) + sd.ring_base;
   const int n_live = kTable ? s_n_live : 0;
   Fetched<T> fetched;
-  RegContext<T, kTable, kFetch> ctx{cur, prm, ps, kUniform ? s_res : lres, (kUniform ? s_res : lres) + kPairs, s_S,
+  RegContext<T, kTable, kFetch, kCluster> ctx{cur, prm, ps, kUniform ? s_res : lres, (kUniform ? s_res : lres) + kPairs, s_S,
                                     s_rows, ring, static_cast<int>(step), nbr, nnbr, nb[0] | (nb[1] << 16),
                                     nb[2] | (nb[3] << 16), nb[4] | (nb[5] << 16),
                                     nnbr > 0 ? T(1) / static_cast<T>(nnbr) : T(0), n, cell, &err, &fetched};
@@ -841,6 +879,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
   double age = pg.age;
   bool dropped = false;
   const int steps_per_chunk = sd.steps_per_chunk;
+  bool folds = false, checks = false;  // analyses that look across a cluster's CTAs
+  if (kCluster)
+    for (int i = 0; i < a.n_analyses; ++i) {
+      folds = folds || a.analyses[i].kind == kBasic;
+      checks = checks || a.analyses[i].kind == kConcCheck;
+    }
 
   for (; chunk < chunk_end; ++chunk) {
     // ---- analyses sample the state at `age` (measurement/base.ipp:4-9)
@@ -851,12 +895,31 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
         if (row >= 0)
           s_vals[row * blk + c] = static_cast<double>(cur[sp]) - (kKahan ? static_cast<double>(comp[sp]) : 0.0);
       }
-      __syncthreads();
-      const bool bad = analyses_sample(a, anl, SmemVals{s_vals, blk}, c, c, n + blk, n, age, s_samples);
+      if (kCluster && folds) {
+        cluster_barrier();
+      } else {
+        __syncthreads();
+      }
+      const SmemVals vals{s_vals, blk, first};
+      bool bad;
+      if constexpr (kCluster)
+        bad = analyses_sample(a, anl, vals, ClusterVals{s_vals, blk}, rank == 0, c, first + c, n + blk, n, age, s_samples);
+      else
+        bad = analyses_sample(a, anl, vals, vals, true, c, c, n + blk, n, age, s_samples);
       if (bad) atomicOr(&s_flags, 1);
-      __syncthreads();
-      if (c < a.n_analyses) s_samples[c] = anl[a.analyses[c].off];
-      if (s_flags & 1) {
+      // a check may drop the set for every CTA; without steps the sampled
+      // state must outlive the folds
+      if (kCluster && (checks || steps_per_chunk == 0)) {
+        cluster_barrier();
+      } else {
+        __syncthreads();
+      }
+      // the counters that the analyses advance in the set's block
+      if (c < a.n_analyses && !(age < a.analyses[c].t0 || age >= a.analyses[c].t1)) s_samples[c] += 1.0;
+      int flags = s_flags;
+      if (kCluster && checks)
+        for (int k = 0; k < ranks; ++k) flags |= *cg::this_cluster().map_shared_rank(&s_flags, k);
+      if (flags & 1) {
         dropped = true;
         break;
       }
@@ -919,14 +982,18 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
         for (int sp = 0; sp < kNS; ++sp) {
           if (kTable) {
             const int w = at[2 * kPairs + sp];
-            if (w >= 0) ring[w + c] = nxt[sp];
+            if (w >= 0) ring[w + cell] = nxt[sp];
           } else {
             const int2 r = s_rows[sp];
-            if (r.x >= 0) ring[((ctx.step + 1) & r.x) * n + r.y + c] = nxt[sp];
+            if (r.x >= 0) ring[((ctx.step + 1) & r.x) * n + r.y + cell] = nxt[sp];
           }
         }
       }
-      __syncthreads();
+      if (kCluster) {
+        cluster_barrier();
+      } else {
+        __syncthreads();
+      }
       ctx.step += 1;
       if (active) {
 #pragma unroll
@@ -941,23 +1008,31 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
   if (active) {
 #pragma unroll
     for (int sp = 0; sp < kNS; ++sp) {
-      state[static_cast<size_t>(sp) * n + c] = cur[sp];
-      if (kKahan) state[static_cast<size_t>(kNS + sp) * n + c] = comp[sp];
+      state[static_cast<size_t>(sp) * n + cell] = cur[sp];
+      if (kKahan) state[static_cast<size_t>(kNS + sp) * n + cell] = comp[sp];
     }
   }
   if (err) atomicOr(&s_flags, err << 1);
-  // pre-finalize sample counters, read before any thread finalizes
-  if (c < a.n_analyses) s_samples[c] = anl[a.analyses[c].off];
-  __syncthreads();
-  const int status = pg.status | (dropped ? kSetDropped : 0) | (s_flags >> 1);
+  int flags;
+  if (kCluster) {
+    // (every CTA has also read the set's progress before rank 0 writes it)
+    cluster_barrier();
+    flags = 0;
+    for (int k = 0; k < ranks; ++k) flags |= *cg::this_cluster().map_shared_rank(&s_flags, k);
+    cluster_barrier();
+  } else {
+    __syncthreads();
+    flags = s_flags;
+  }
+  const int status = pg.status | (dropped ? kSetDropped : 0) | (flags >> 1);
   const bool finish = !dropped && chunk >= sd.n_chunks;
   if (finish) {
     for (int ai = 0; ai < a.n_analyses; ++ai) {
       const AnalysisDesc& A = a.analyses[ai];
-      if (A.kind == kOscillation) osc_cell_finalize(anl + A.off, A, c, s_samples[ai]);
+      if (A.kind == kOscillation) osc_cell_finalize(anl + A.off, A, first + c, s_samples[ai]);
     }
   }
-  if (c == 0) {
+  if (first + c == 0) {
     SetProgress out = pg;
     out.step = step;
     out.chunk = chunk;
@@ -1068,8 +1143,8 @@ __global__ void __launch_bounds__(256, 2) dense_step_mem_kernel(const StepArgs a
         }
       }
       __syncthreads();
-      const bool bad =
-          analyses_sample(a, anl, RingVals<T>{s_rows, kKahan ? s_crows : nullptr}, tid, tid, blk, n, age, s_samples);
+      const RingVals<T> vals{s_rows, kKahan ? s_crows : nullptr};
+      const bool bad = analyses_sample(a, anl, vals, vals, true, tid, tid, blk, n, age, s_samples);
       if (bad) atomicOr(&s_flags, 1);
       __syncthreads();
       if (tid < a.n_analyses) s_samples[tid] = anl[a.analyses[tid].off];
@@ -1424,8 +1499,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_wave_kernel(c
         }
       }
       __syncthreads();
-      const bool bad =
-          analyses_sample(a, anl, RingVals<T>{s_rows, kKahan ? s_crows : nullptr}, tid, tid, blk, n, age, s_samples);
+      const RingVals<T> vals{s_rows, kKahan ? s_crows : nullptr};
+      const bool bad = analyses_sample(a, anl, vals, vals, true, tid, tid, blk, n, age, s_samples);
       if (bad) atomicOr(&s_flags, 1);
       __syncthreads();
       if (tid < a.n_analyses) s_samples[tid] = anl[a.analyses[tid].off];
@@ -1589,7 +1664,7 @@ __global__ void dense_import_kernel(const StepArgs a, int set, const double* sam
   bool dropped = false;
   for (; k < num_samples; ++k) {
     const ImportVals vals{samples + static_cast<size_t>(k) * a.n_vals * n, n};
-    const bool bad = analyses_sample(a, anl, vals, tid, tid, blk, n, age, s_samples);
+    const bool bad = analyses_sample(a, anl, vals, vals, true, tid, tid, blk, n, age, s_samples);
     if (bad) atomicOr(&s_flags, 1);
     __syncthreads();
     if (tid < a.n_analyses) s_samples[tid] = anl[a.analyses[tid].off];
@@ -1695,7 +1770,7 @@ inline int sm_count() {
 // Launchers, named by the including translation unit's precision suffix.
 #define DENSE_B200_STEP_VARIANT(T, KAHAN, THREADS, BLOCKS, UNIFORM, SMEM_CAP)                     \
   {                                                                                             \
-    auto k = dense_step_kernel<T, KAHAN, THREADS, BLOCKS, UNIFORM>;                             \
+    auto k = dense_step_kernel<T, KAHAN, THREADS, BLOCKS, UNIFORM, false>;                      \
     static bool configured = false;                                                             \
     if (!configured) {                                                                          \
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP); \
@@ -1704,6 +1779,19 @@ inline int sm_count() {
     }                                                                                           \
     k<<<n_sets, a.block_threads, smem, s>>>(a, set_list);                                       \
     return cudaGetLastError();                                                                  \
+  }
+
+#define DENSE_B200_CLUSTER_VARIANT(T, KAHAN, BLOCKS, UNIFORM)                                    \
+  {                                                                                             \
+    auto k = dense_step_kernel<T, KAHAN, 256, BLOCKS, UNIFORM, true>;                            \
+    static bool configured = false;                                                             \
+    if (!configured) {                                                                          \
+      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmem); \
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); \
+      if (e != cudaSuccess) return e;                                                           \
+      configured = true;                                                                        \
+    }                                                                                           \
+    return cudaLaunchKernelEx(&cfg, k, a, set_list);                                            \
   }
 
 #define DENSE_B200_WAVE_VARIANT(T, KAHAN, UNIFORM, THREADS, MINB, SHARED)                       \
@@ -1750,6 +1838,29 @@ inline int sm_count() {
       else DENSE_B200_WAVE_VARIANT(T, KAHAN, false, 256, 2, false)                              \
     }                                                                                           \
     return cudaGetLastError();                                                                  \
+  }                                                                                             \
+  cudaError_t launch_step_cluster_##SUFFIX(const StepArgs& a, const int* set_list, int n_sets, int threads, \
+                                           int ranks, cudaStream_t s) {                          \
+    if (n_sets <= 0) return cudaSuccess;                                                        \
+    cudaLaunchAttribute attr{};                                                                 \
+    attr.id = cudaLaunchAttributeClusterDimension;                                              \
+    attr.val.clusterDim.x = ranks;                                                              \
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;                                          \
+    cudaLaunchConfig_t cfg{};                                                                   \
+    cfg.gridDim = dim3(n_sets * ranks);                                                         \
+    cfg.blockDim = dim3(threads);                                                               \
+    cfg.dynamicSmemBytes = a.n_analyses > 0 ? sizeof(double) * a.n_vals * threads : 0;          \
+    cfg.stream = s;                                                                             \
+    cfg.attrs = &attr;                                                                          \
+    cfg.numAttrs = 1;                                                                           \
+    /* as below: two CTAs per SM (128 registers) past one wave */                               \
+    if (n_sets * ranks > sm_count()) {                                                          \
+      if (a.uniform_params) DENSE_B200_CLUSTER_VARIANT(T, KAHAN, 2, true)                        \
+      else DENSE_B200_CLUSTER_VARIANT(T, KAHAN, 2, false)                                         \
+    } else {                                                                                    \
+      if (a.uniform_params) DENSE_B200_CLUSTER_VARIANT(T, KAHAN, 1, true)                        \
+      else DENSE_B200_CLUSTER_VARIANT(T, KAHAN, 1, false)                                         \
+    }                                                                                           \
   }                                                                                             \
   cudaError_t launch_step_##SUFFIX(const StepArgs& a, const int* set_list, int n_sets, size_t smem, \
                                    cudaStream_t s) {                                            \

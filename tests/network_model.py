@@ -73,7 +73,8 @@ def engine_states(model, sets, dt, interval, analyses=(), precision=0, chunks=No
     for i in range(len(sets)):
         r = {"state": b.state(i), "status": int(status[i])}
         for k, a in enumerate(analyses):
-            r[k] = b.basic(k, i) if a.kind == E.BASIC else b.oscillation(k, i)
+            if a.kind in (E.BASIC, E.OSCILLATION):
+                r[k] = b.basic(k, i) if a.kind == E.BASIC else b.oscillation(k, i)
         out.append(r)
     b.close()
     return out
