@@ -611,7 +611,7 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
     for (int i = 0; i < A.nsp; ++i)
       if (!sampled[A.sp[i]]) {
         sampled[A.sp[i]] = true;
-        sample_bytes += sizeof(double) * kStepThreads;
+        sample_bytes += sizeof(double) * (kStepThreads + kValsPad);
       }
   std::vector<double> cp;
   for (int s = 0; s < num_sets; ++s) {
@@ -849,7 +849,7 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
   for (int i = 0; i < a.n_analyses; ++i)
     for (int k = 0; k < a.analyses[i].nsp; ++k) a.analyses[i].slot[k] = a.val_slot[a.analyses[i].sp[k]];
   e->analyses.assign(a.analyses, a.analyses + a.n_analyses);
-  size_t smem = a.n_analyses > 0 ? sizeof(double) * a.n_vals * a.block_threads : 0;
+  size_t smem = a.n_analyses > 0 ? sizeof(double) * a.n_vals * (a.block_threads + kValsPad) : 0;
   const size_t csr_bytes = sizeof(int) * max_edges;
   const size_t smem_cap = a.block_threads <= 224 ? 100000 : 200000;
   a.csr_in_smem = smem + csr_bytes <= smem_cap ? 1 : 0;

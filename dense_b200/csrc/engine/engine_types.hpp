@@ -19,6 +19,7 @@ constexpr int kNP = NUM_PARAMS;
 constexpr int kMaxAnalyses = 8;
 constexpr int kStepThreads = 256;  // register kernel: one thread per cell, one CTA per set
 constexpr int kMaxCells = 65536;   // memory kernel: cells per set
+constexpr int kValsPad = 2;        // register kernel: doubles between the rows of the sampled state
 constexpr int kMaxCluster = 16;    // register kernel: CTAs a set's cells may be spread over (above the portable 8)
 constexpr int kClusterSmem = 100000;  // dynamic shared memory of such a CTA (two per SM)
 constexpr int64_t kMaxRegisterRing = 1 << 25;  // register kernel: elements of one set's history rings

@@ -368,7 +368,7 @@ constexpr bool kRowTables = kPairs > 0 && kPairs <= 1024;
 // BasicAnalysis::update (basic.ipp:22-36), per-cell part: thread c updates
 // its own column.  std::min(x, m) = (m < x) ? m : x, std::max(x, M) =
 // (x < M) ? M : x, NaN behaviour kept.
-template <typename Vals>
+template <int kAhead, typename Vals>
 __device__ __forceinline__ void basic_cell_update(double* st, const AnalysisDesc& A, const Vals& vals, int c) {
   const int n = A.nsp;
   const int m = A.cmax - A.cmin;
@@ -377,13 +377,28 @@ __device__ __forceinline__ void basic_cell_update(double* st, const AnalysisDesc
   double* cmaxs = cmins + static_cast<size_t>(m) * n;
   double* csums = cmaxs + static_cast<size_t>(m) * n;
   const int cc = c - A.cmin;
-  for (int i = 0; i < n; ++i) {
-    const double x = vals(A.slot[i], c);
-    const size_t k = static_cast<size_t>(i) * m + cc;
-    const double mn = cmins[k], mx = cmaxs[k];
-    cmins[k] = (mn < x) ? mn : x;
-    cmaxs[k] = (x < mx) ? mx : x;
-    csums[k] = csums[k] + x;
+  // kAhead species' loads at once: one after the other, each waits for the
+  // loads of a line of its own
+  for (int i0 = 0; i0 < n; i0 += kAhead) {
+    const int live = min(kAhead, n - i0);
+    double mn[kAhead], mx[kAhead], sm[kAhead], x[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      if (j >= live) continue;
+      const size_t k = static_cast<size_t>(i0 + j) * m + cc;
+      mn[j] = cmins[k];
+      mx[j] = cmaxs[k];
+      sm[j] = csums[k];
+      x[j] = vals(A.slot[i0 + j], c);
+    }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      if (j >= live) continue;
+      const size_t k = static_cast<size_t>(i0 + j) * m + cc;
+      cmins[k] = (mn[j] < x[j]) ? mn[j] : x[j];
+      cmaxs[k] = (x[j] < mx[j]) ? mx[j] : x[j];
+      csums[k] = sm[j] + x[j];
+    }
   }
 }
 
@@ -391,17 +406,25 @@ __device__ __forceinline__ void basic_cell_update(double* st, const AnalysisDesc
 // cell order, as DENSE's loop does (cells outer, species inner; each
 // species' accumulator only sees its own values, so per-species folds in
 // cell order give the same results bit for bit).
-template <typename Vals>
+template <int kAhead, typename Vals>
 __device__ __forceinline__ void basic_range_fold(double* st, const AnalysisDesc& A, const Vals& vals, int lane) {
   const int n = A.nsp;
   for (int i = lane; i < n; i += 32) {
     double mn = st[i], mx = st[n + i], sm = st[2 * n + i];
-    for (int c = A.cmin; c < A.cmax; ++c) {
-      const double x = vals(A.slot[i], c);
+    auto take = [&](double x) {
       mn = (mn < x) ? mn : x;
       mx = (x < mx) ? mx : x;
       sm = sm + x;
+    };
+    int c = A.cmin;
+    for (; c + 2 * kAhead <= A.cmax; c += 2 * kAhead) {  // loads ahead of the three chains
+      double x[2 * kAhead];
+#pragma unroll
+      for (int j = 0; j < 2 * kAhead; ++j) x[j] = vals(A.slot[i], c + j);
+#pragma unroll
+      for (int j = 0; j < 2 * kAhead; ++j) take(x[j]);
     }
+    for (; c < A.cmax; ++c) take(vals(A.slot[i], c));
     st[i] = mn;
     st[n + i] = mx;
     st[2 * n + i] = sm;
@@ -422,8 +445,8 @@ struct OscRef {
 // Queue::getSize, (size + end - start) % size + 1.  With end in [-1, size)
 // and start in [0, size) the dividend lies in [0, 2 * size), so one
 // conditional subtraction gives the same remainder.
-__device__ __forceinline__ long q_size(long start, long end, long size) {
-  const long x = size + end - start;
+__device__ __forceinline__ int q_size(int start, int end, int size) {
+  const int x = size + end - start;
   return (x < size ? x : x - size) + 1;
 }
 
@@ -464,27 +487,16 @@ __device__ __forceinline__ void osc_add_crit(const OscRef& o, double t, double c
   o.f(kOscNcrit) += 1.0;
 }
 
-// The queue part of one (species, cell), held in registers while a sample
-// is processed; loaded and stored as one batch of independent accesses.
-struct OscQueue {
-  long start, end, current, live;
-  long same;  // the newest `same` values are equal (so the window is flat when same >= live)
-  __device__ __forceinline__ void load(const OscRef& o) {
-    const double s0 = o.f(kOscStart), e0 = o.f(kOscEnd), c0 = o.f(kOscCurrent), l0 = o.f(kOscLive);
-    const double m0 = o.f(kOscSame);
-    start = static_cast<long>(s0);
-    end = static_cast<long>(e0);
-    current = static_cast<long>(c0);
-    live = static_cast<long>(l0);
-    same = static_cast<long>(m0);
-  }
-  __device__ __forceinline__ void store(const OscRef& o) const {
-    o.f(kOscStart) = static_cast<double>(start);
-    o.f(kOscEnd) = static_cast<double>(end);
-    o.f(kOscCurrent) = static_cast<double>(current);
-    o.f(kOscLive) = static_cast<double>(live);
-    o.f(kOscSame) = static_cast<double>(same);
-  }
+// The queue indices of one (species, cell).  They follow from the number of
+// samples alone, so every cell of a species has the same: during a launch
+// each CTA keeps one copy per (analysis, species) in shared memory, and the
+// cells' own fields are read when it begins and written when it ends
+// (osc_load_indices, osc_store_indices).  With eight index fields read and
+// written per cell, species and sample, 100 samples of two species in 160
+// cells took 0.37 ms beside 1000 steps' 2.4 ms, and 0.33 ms so; over 1024
+// sets on a full GPU 1.24 and 1.04 ms.
+struct __align__(16) OscIndex {
+  int start, end, current, live;
   // Queue::dequeue (the value leaves DENSE's multiset too)
   __device__ __forceinline__ void dequeue(int w) {
     start = (start == w - 1) ? 0 : start + 1;
@@ -493,6 +505,39 @@ struct OscQueue {
       if (current == w) current = 0;
     }
     live -= 1;
+  }
+  // A sample's enqueue, and dequeue of a full window; whether the window is
+  // still too short to be looked at.
+  __device__ __forceinline__ bool sample(int w) {
+    end = (end == w - 1) ? 0 : end + 1;
+    live += 1;
+    if (2 * q_size(start, end, w) >= w) {
+      current = current + 1;
+      if (current == w) current = 0;
+    }
+    if (q_size(start, end, w) == w) dequeue(w);
+    return q_size(start, end, w) < (w - 1) / 2;
+  }
+};
+
+// With the run of equal newest values, which is each cell's own: the newest
+// `same` values are equal (so the window is flat when same >= live).
+struct OscQueue : OscIndex {
+  int same;
+  __device__ __forceinline__ void load(const OscRef& o) {
+    const double s0 = o.f(kOscStart), e0 = o.f(kOscEnd), c0 = o.f(kOscCurrent), l0 = o.f(kOscLive);
+    const double m0 = o.f(kOscSame);
+    start = static_cast<int>(s0);
+    end = static_cast<int>(e0);
+    current = static_cast<int>(c0);
+    live = static_cast<int>(l0);
+    same = static_cast<int>(m0);
+  }
+  __device__ __forceinline__ void store(const OscRef& o) const {
+    o.f(kOscStart) = static_cast<double>(start);
+    o.f(kOscEnd) = static_cast<double>(end);
+    o.f(kOscCurrent) = static_cast<double>(current);
+    o.f(kOscLive) = static_cast<double>(live);
   }
 };
 
@@ -523,8 +568,8 @@ __device__ __forceinline__ void osc_check(const OscRef& o, const OscQueue& q, co
     osc_add_crit(o, t, mid, false);
     return;
   }
-  long lo = q.start, hi = q.end;  // oldest and newest live slots
-  long left = q.live;             // live values not yet looked at
+  int lo = q.start, hi = q.end;  // oldest and newest live slots
+  int left = q.live;             // live values not yet looked at
   while (left > 0 && !(above && below)) {
     // slots past the live values hold mid, which is neither above nor below
     double x[8];
@@ -563,10 +608,11 @@ __device__ __forceinline__ double* osc_window(double* st, const AnalysisDesc& A,
 
 // OscillationAnalysis::update / get_peaks_and_troughs (oscillation.ipp:
 // 86-103, 154-160) for thread c's cell, species in observation order,
-// stopping at the first species whose window is still short.
+// stopping at the first species whose window is still short.  `index`: the
+// species' queue indices before this sample.
 template <typename Vals>
 __device__ __forceinline__ void osc_cell_update(double* st, const AnalysisDesc& A, const Vals& vals, int c,
-                                                double samples) {
+                                                double samples, const OscIndex* index) {
   if (c < A.cmin || c >= A.cmax) return;
   const int n = A.nsp, m = A.cmax - A.cmin, w = A.range_steps + 1;
   const int cc = c - A.cmin;
@@ -575,23 +621,52 @@ __device__ __forceinline__ void osc_cell_update(double* st, const AnalysisDesc& 
     double* win = osc_window(st, A, i, cc);
     const double added = vals(A.slot[i], c);
     OscQueue q;
-    q.load(o);
+    static_cast<OscIndex&>(q) = index[i];
     // the run of equal newest values (NaN equals nothing)
+    const double run = o.f(kOscSame);
     const double newest = q.live > 0 ? win[static_cast<size_t>(q.end) * m] : added;
-    q.same = (q.live > 0 && newest == added) ? q.same + 1 : (added == added ? 1 : 0);
+    q.same = (q.live > 0 && newest == added) ? static_cast<int>(run) + 1 : (added == added ? 1 : 0);
     // Queue::enqueue; the multiset gains `added`
-    q.end = (q.end == w - 1) ? 0 : q.end + 1;
+    const bool stop = q.sample(w);
     win[static_cast<size_t>(q.end) * m] = added;
-    q.live += 1;
-    if (2 * q_size(q.start, q.end, w) >= w) {
-      q.current = q.current + 1;
-      if (q.current == w) q.current = 0;
-    }
-    if (q_size(q.start, q.end, w) == A.range_steps + 1) q.dequeue(w);
-    const bool stop = q_size(q.start, q.end, w) < A.range_steps / 2;
+    o.f(kOscSame) = static_cast<double>(q.same);
     if (!stop) osc_check(o, q, win, m, w, samples, A);
-    q.store(o);
     if (stop) break;
+  }
+}
+
+// One thread per analysis: its species' indices past a sample.
+__device__ __forceinline__ void osc_advance(const AnalysisDesc& A, OscIndex* index) {
+  for (int i = 0; i < A.nsp; ++i)
+    if (index[i].sample(A.range_steps + 1)) break;
+}
+
+// The indices of every oscillation analysis, from (to) the fields of its
+// first (of every) cell.
+__device__ __forceinline__ void osc_load_indices(const StepArgs& a, double* anl, OscIndex (*index)[kNS], int tid,
+                                                 int threads) {
+  for (int k = tid; k < a.n_analyses * kNS; k += threads) {
+    const AnalysisDesc& A = a.analyses[k / kNS];
+    const int i = k % kNS;
+    if (A.kind != kOscillation || i >= A.nsp || A.cmax <= A.cmin) continue;
+    OscQueue q;
+    q.load(osc_ref(anl + A.off, A, i, 0));
+    index[k / kNS][i] = q;
+  }
+}
+__device__ __forceinline__ void osc_store_indices(const StepArgs& a, double* anl, const OscIndex (*index)[kNS], int c0,
+                                                  int stride, int n) {
+  for (int ai = 0; ai < a.n_analyses; ++ai) {
+    const AnalysisDesc& A = a.analyses[ai];
+    if (A.kind != kOscillation) continue;
+    for (int c = c0; c < n; c += stride) {
+      if (c < A.cmin || c >= A.cmax) continue;
+      for (int i = 0; i < A.nsp; ++i) {
+        OscQueue q;
+        static_cast<OscIndex&>(q) = index[ai][i];
+        q.store(osc_ref(anl + A.off, A, i, c - A.cmin));
+      }
+    }
   }
 }
 
@@ -631,9 +706,9 @@ __device__ __forceinline__ void osc_cell_finalize(double* st, const AnalysisDesc
 // the register kernel, or the lag-0 rows of the rings in the memory kernel.
 struct SmemVals {
   const double* base;  // of the CTA's first cell
-  int blk;
+  int pitch;           // of the rows
   int first;
-  __device__ __forceinline__ double operator()(int slot, int cell) const { return base[slot * blk + cell - first]; }
+  __device__ __forceinline__ double operator()(int slot, int cell) const { return base[slot * pitch + cell - first]; }
 };
 
 // The same over a cluster whose CTAs hold `blk` cells each.
@@ -642,7 +717,7 @@ struct ClusterVals {
   int blk;
   __device__ __forceinline__ double operator()(int slot, int cell) const {
     const int rank = cell / blk;
-    return cooperative_groups::this_cluster().map_shared_rank(base, rank)[slot * blk + cell - rank * blk];
+    return cooperative_groups::this_cluster().map_shared_rank(base, rank)[slot * (blk + kValsPad) + cell - rank * blk];
   }
 };
 
@@ -669,10 +744,10 @@ struct RingVals {
 // of the set; with `lead` this CTA does what is done once per set (tid 0,
 // and the whole-range folds of warp 0).  Returns whether a concentration
 // check failed for one of the thread's cells.
-template <typename Vals, typename Fold>
+template <int kAhead, typename Vals, typename Fold>
 __device__ __forceinline__ bool analyses_sample(const StepArgs& a, double* anl, const Vals& vals, const Fold& fold,
                                                 bool lead, int tid, int c0, int stride, int n, double age,
-                                                const double* samples) {
+                                                const double* samples, const OscIndex (*index)[kNS]) {
   bool bad = false;
   for (int ai = 0; ai < a.n_analyses; ++ai) {
     const AnalysisDesc& A = a.analyses[ai];
@@ -681,13 +756,13 @@ __device__ __forceinline__ bool analyses_sample(const StepArgs& a, double* anl, 
     if (A.kind == kBasic) {
       if (lead && tid == 0) st[3 * A.nsp + 1] = age;
       if (!in_range) continue;
-      for (int c = c0; c < n; c += stride) basic_cell_update(st, A, vals, c);
-      if (lead && tid < 32) basic_range_fold(st, A, fold, tid);
+      for (int c = c0; c < n; c += stride) basic_cell_update<kAhead>(st, A, vals, c);
+      if (lead && tid < 32) basic_range_fold<kAhead>(st, A, fold, tid);
       if (lead && tid == 0) st[3 * A.nsp] += 1.0;
     } else if (A.kind == kOscillation) {
       if (lead && tid == 0) st[1] = age;
       if (!in_range) continue;
-      for (int c = c0; c < n; c += stride) osc_cell_update(st, A, vals, c, samples[ai]);
+      for (int c = c0; c < n; c += stride) osc_cell_update(st, A, vals, c, samples[ai], index[ai]);
       if (lead && tid == 0) st[0] = samples[ai] + 1.0;
     } else if (A.kind == kTrajectory) {
       // csvw_sim::update (io/csvw_sim.ipp:17-91): every observed species
@@ -737,25 +812,34 @@ __device__ __forceinline__ bool analyses_sample(const StepArgs& a, double* anl, 
 // of three that the GPU holds at once, 1.02 ms (5.1 us a step, of which the
 // cluster barrier and the release of the rows written before it are a
 // quarter).
+//
+// kAhead: species a sample's Basic analysis loads at once.  With one CTA per
+// SM the sample is a chain of loads and there are registers for four (160
+// cells, 14 species, 100 samples and 1000 steps: 3.93 ms with one at a
+// time, 3.59 with four); with two the loads' registers are taken from the
+// steps (1024 such sets: 13.3 ms with one, 13.8 with two, 14.8 with four).
 template <typename T, bool kKahan, int kThreads, int kMinBlocks, bool kUniform, bool kCluster>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const StepArgs a, const int* set_list) {
-  // dynamic shared memory: sampled state [n_vals][blockDim] (doubles, only
-  // with analyses) | the set's neighbour ids
+  // dynamic shared memory: sampled state [n_vals][blockDim + 2] (doubles,
+  // only with analyses; a whole-range fold reads one cell of every species
+  // at once, which the 2 spread over the banks) | the set's neighbour ids
   extern __shared__ double s_dyn[];
   double* s_vals = s_dyn;
   constexpr bool kTable = kUniform && kRowTables;
+  constexpr int kAhead = kMinBlocks == 1 ? 4 : 1;
   __shared__ int s_S[kNS];
   __shared__ int2 s_rows[kNS];  // staged depth - 1 (-1: none), ring offset
   __shared__ __align__(16) T s_prm[kNP];
   __shared__ int s_flags;
   __shared__ double s_samples[kMaxAnalyses];
+  __shared__ OscIndex s_index[kMaxAnalyses][kNS];
   // resolved reads (own, then neighbour); kTable: their row offsets of this
   // step and the next, then the rows written, and the entries that advance
   constexpr int kReads = kUniform ? 2 * kPairs : 0;
   constexpr int kEntries = kTable ? 2 * kPairs + kNS : 0;
   __shared__ int s_res[kReads > 0 ? kReads : 1];
   __shared__ int s_at[2][kEntries > 0 ? kEntries : 1];
-  __shared__ unsigned short s_live[kEntries > 0 ? kEntries : 1];
+  __shared__ int4 s_live[kEntries > 0 ? kEntries : 1];  // {lag (-1: the row written), depth - 1, ring offset, entry}
   __shared__ int s_n_live;
 
   namespace cg = cooperative_groups;
@@ -787,6 +871,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
   }
   double* anl = a.anl + sd.anl_base;
   if (c < a.n_analyses) s_samples[c] = anl[a.analyses[c].off];
+  osc_load_indices(a, anl, s_index, c, blk);
   __syncthreads();
 
   const int cell = active ? first + c : 0;
@@ -813,13 +898,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
       }
     }
   }
-  // one entry of the row table: the offset of the row it names at step t
-  auto row_offset = [&](int e, int t) {
-    const bool write = e >= 2 * kPairs;
-    const int2 r = s_rows[write ? e - 2 * kPairs : e % kNS];
-    const int lag = write ? -1 : s_res[e];
-    return ((t - lag) & r.x) * n + r.y;
-  };
   if (kTable) {
     __syncthreads();
     for (int e = c; e < kEntries; e += blk) {
@@ -832,9 +910,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
         live = e < kPairs ? res > 0 : res >= 0;
         at = res < 0 ? kReadChecked : kReadLag0;
       }
-      if (live) s_live[atomicAdd(&s_n_live, 1)] = static_cast<unsigned short>(e);
+      if (live) {
+        const bool write = e >= 2 * kPairs;
+        const int2 r = s_rows[write ? e - 2 * kPairs : e % kNS];
+        const int lag = write ? -1 : s_res[e];
+        s_live[atomicAdd(&s_n_live, 1)] = make_int4(lag, r.x, r.y, e);
+        at = ((static_cast<int>(step) - lag) & r.x) * n + r.y;
+      }
       s_at[0][e] = s_at[1][e] = at;
-      if (live) s_at[step & 1][e] = row_offset(e, static_cast<int>(step));
     }
   }
 
@@ -855,7 +938,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
   for (int e = 0; e < 6; ++e) nb[e] = e < nnbr ? static_cast<uint32_t>(nbr[e]) : 0u;
   if (!kCluster && a.csr_in_smem) {
     // the set's neighbour ids, [edges], in shared memory
-    int* s_csr = reinterpret_cast<int*>(s_dyn + (a.n_analyses > 0 ? a.n_vals * blk : 0));
+    int* s_csr = reinterpret_cast<int*>(s_dyn + (a.n_analyses > 0 ? a.n_vals * (blk + kValsPad) : 0));
     const int e0 = nbr_off[0], ne = nbr_off[n] - e0;
     for (int e = c; e < ne; e += blk) s_csr[e] = a.nbr_idx[e0 + e];
     nbr = s_csr + (nb0 - e0);
@@ -892,20 +975,22 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
 #pragma unroll
       for (int sp = 0; sp < kNS; ++sp) {
         const int row = a.val_slot[sp];
-        if (row >= 0)
-          s_vals[row * blk + c] = static_cast<double>(cur[sp]) - (kKahan ? static_cast<double>(comp[sp]) : 0.0);
+        if (row < 0) continue;
+        s_vals[row * (blk + kValsPad) + c] =
+            static_cast<double>(cur[sp]) - (kKahan ? static_cast<double>(comp[sp]) : 0.0);
       }
       if (kCluster && folds) {
         cluster_barrier();
       } else {
         __syncthreads();
       }
-      const SmemVals vals{s_vals, blk, first};
+      const SmemVals vals{s_vals, blk + kValsPad, first};
       bool bad;
       if constexpr (kCluster)
-        bad = analyses_sample(a, anl, vals, ClusterVals{s_vals, blk}, rank == 0, c, first + c, n + blk, n, age, s_samples);
+        bad = analyses_sample<kAhead>(a, anl, vals, ClusterVals{s_vals, blk}, rank == 0, c, first + c, n + blk, n,
+                                      age, s_samples, s_index);
       else
-        bad = analyses_sample(a, anl, vals, vals, true, c, c, n + blk, n, age, s_samples);
+        bad = analyses_sample<kAhead>(a, anl, vals, vals, true, c, c, n + blk, n, age, s_samples, s_index);
       if (bad) atomicOr(&s_flags, 1);
       // a check may drop the set for every CTA; without steps the sampled
       // state must outlive the folds
@@ -914,8 +999,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
       } else {
         __syncthreads();
       }
-      // the counters that the analyses advance in the set's block
-      if (c < a.n_analyses && !(age < a.analyses[c].t0 || age >= a.analyses[c].t1)) s_samples[c] += 1.0;
+      // the counters that the analyses advance in the set's block, and the
+      // queue indices
+      if (c < a.n_analyses && !(age < a.analyses[c].t0 || age >= a.analyses[c].t1)) {
+        s_samples[c] += 1.0;
+        if (a.analyses[c].kind == kOscillation) osc_advance(a.analyses[c], s_index[c]);
+      }
       int flags = s_flags;
       if (kCluster && checks)
         for (int k = 0; k < ranks; ++k) flags |= *cg::this_cluster().map_shared_rank(&s_flags, k);
@@ -935,8 +1024,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
         // the next step's rows
         int* next = s_at[(ctx.step + 1) & 1];
         for (int i = c; i < n_live; i += blk) {
-          const int e = s_live[i];
-          next[e] = row_offset(e, ctx.step + 1);
+          const int4 e = s_live[i];
+          next[e.w] = ((ctx.step + 1 - e.x) & e.y) * n + e.z;
         }
       }
       if (active) {
@@ -1024,6 +1113,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
     __syncthreads();
     flags = s_flags;
   }
+  osc_store_indices(a, anl, s_index, first + c, n + blk, n);
   const int status = pg.status | (dropped ? kSetDropped : 0) | (flags >> 1);
   const bool finish = !dropped && chunk >= sd.n_chunks;
   if (finish) {
@@ -1086,6 +1176,7 @@ __global__ void __launch_bounds__(256, 2) dense_step_mem_kernel(const StepArgs a
   __shared__ T s_prm[kNP];
   __shared__ int s_flags;
   __shared__ double s_samples[kMaxAnalyses];
+  __shared__ OscIndex s_index[kMaxAnalyses][kNS];
   __shared__ int s_olag[kND > 0 ? kND * kNS : 1], s_nlag[kND > 0 ? kND * kNS : 1];
   __shared__ T* s_rows[kNS];
   __shared__ T* s_crows[kNS];
@@ -1112,6 +1203,7 @@ __global__ void __launch_bounds__(256, 2) dense_step_mem_kernel(const StepArgs a
   if (tid == 0) s_flags = 0;
   double* anl = a.anl + sd.anl_base;
   if (tid < a.n_analyses) s_samples[tid] = anl[a.analyses[tid].off];
+  osc_load_indices(a, anl, s_index, tid, blk);
   __syncthreads();
   if (kUniform) fill_lag_tables(s_prm, s_S, s_mask, s_olag, s_nlag, tid, blk);
   __syncthreads();
@@ -1144,10 +1236,14 @@ __global__ void __launch_bounds__(256, 2) dense_step_mem_kernel(const StepArgs a
       }
       __syncthreads();
       const RingVals<T> vals{s_rows, kKahan ? s_crows : nullptr};
-      const bool bad = analyses_sample(a, anl, vals, vals, true, tid, tid, blk, n, age, s_samples);
+      const bool bad = analyses_sample<1>(a, anl, vals, vals, true, tid, tid, blk, n, age, s_samples, s_index);
       if (bad) atomicOr(&s_flags, 1);
       __syncthreads();
-      if (tid < a.n_analyses) s_samples[tid] = anl[a.analyses[tid].off];
+      if (tid < a.n_analyses) {
+        const AnalysisDesc& A = a.analyses[tid];
+        s_samples[tid] = anl[A.off];
+        if (A.kind == kOscillation && !(age < A.t0 || age >= A.t1)) osc_advance(A, s_index[tid]);
+      }
       if (s_flags & 1) {
         dropped = true;
         break;
@@ -1212,6 +1308,7 @@ __global__ void __launch_bounds__(256, 2) dense_step_mem_kernel(const StepArgs a
   if (err) atomicOr(&s_flags, err << 1);
   if (tid < a.n_analyses) s_samples[tid] = anl[a.analyses[tid].off];
   __syncthreads();
+  osc_store_indices(a, anl, s_index, tid, blk, n);
   const int status = pg.status | (dropped ? kSetDropped : 0) | (s_flags >> 1);
   const bool finish = !dropped && chunk >= sd.n_chunks;
   if (finish) {
@@ -1377,6 +1474,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_wave_kernel(c
   __shared__ T s_prm[kNP];
   __shared__ int s_flags;
   __shared__ double s_samples[kMaxAnalyses];
+  __shared__ OscIndex s_index[kMaxAnalyses][kNS];
   __shared__ int s_olag[kND > 0 ? kND * kNS : 1], s_nlag[kND > 0 ? kND * kNS : 1];
   __shared__ T* s_rows[kNS];
   __shared__ T* s_crows[kNS];
@@ -1405,6 +1503,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_wave_kernel(c
   if (tid == 0) s_flags = 0;
   double* anl = a.anl + sd.anl_base;
   if (tid < a.n_analyses) s_samples[tid] = anl[a.analyses[tid].off];
+  osc_load_indices(a, anl, s_index, tid, blk);
 
   // level offsets (16-bit) and cell records: shared, or records global
   const int n_levels = sd.n_levels;
@@ -1500,10 +1599,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_wave_kernel(c
       }
       __syncthreads();
       const RingVals<T> vals{s_rows, kKahan ? s_crows : nullptr};
-      const bool bad = analyses_sample(a, anl, vals, vals, true, tid, tid, blk, n, age, s_samples);
+      const bool bad = analyses_sample<1>(a, anl, vals, vals, true, tid, tid, blk, n, age, s_samples, s_index);
       if (bad) atomicOr(&s_flags, 1);
       __syncthreads();
-      if (tid < a.n_analyses) s_samples[tid] = anl[a.analyses[tid].off];
+      if (tid < a.n_analyses) {
+        const AnalysisDesc& A = a.analyses[tid];
+        s_samples[tid] = anl[A.off];
+        if (A.kind == kOscillation && !(age < A.t0 || age >= A.t1)) osc_advance(A, s_index[tid]);
+      }
       if (s_flags & 1) {
         dropped = true;
         break;
@@ -1614,6 +1717,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_wave_kernel(c
   if (err) atomicOr(&s_flags, err << 1);
   if (tid < a.n_analyses) s_samples[tid] = anl[a.analyses[tid].off];
   __syncthreads();
+  osc_store_indices(a, anl, s_index, tid, blk, n);
   const int status = pg.status | (dropped ? kSetDropped : 0) | (s_flags >> 1);
   const bool finish = !dropped && chunk >= sd.n_chunks;
   if (finish) {
@@ -1651,12 +1755,14 @@ template <typename T>
 __global__ void dense_import_kernel(const StepArgs a, int set, const double* samples, int num_samples,
                                     double time_start) {
   __shared__ double s_samples[kMaxAnalyses];
+  __shared__ OscIndex s_index[kMaxAnalyses][kNS];
   __shared__ int s_flags;
   const SetDesc& sd = a.sets[set];
   const int n = sd.n_cells;
   const int tid = threadIdx.x, blk = blockDim.x;
   double* anl = a.anl + sd.anl_base;
   if (tid < a.n_analyses) s_samples[tid] = anl[a.analyses[tid].off];
+  osc_load_indices(a, anl, s_index, tid, blk);
   if (tid == 0) s_flags = 0;
   __syncthreads();
   double age = time_start;
@@ -1664,17 +1770,23 @@ __global__ void dense_import_kernel(const StepArgs a, int set, const double* sam
   bool dropped = false;
   for (; k < num_samples; ++k) {
     const ImportVals vals{samples + static_cast<size_t>(k) * a.n_vals * n, n};
-    const bool bad = analyses_sample(a, anl, vals, vals, true, tid, tid, blk, n, age, s_samples);
+    const bool bad = analyses_sample<4>(a, anl, vals, vals, true, tid, tid, blk, n, age, s_samples, s_index);
     if (bad) atomicOr(&s_flags, 1);
     __syncthreads();
-    if (tid < a.n_analyses) s_samples[tid] = anl[a.analyses[tid].off];
+    if (tid < a.n_analyses) {
+      const AnalysisDesc& A = a.analyses[tid];
+      s_samples[tid] = anl[A.off];
+      if (A.kind == kOscillation && !(age < A.t0 || age >= A.t1)) osc_advance(A, s_index[tid]);
+    }
     if (s_flags & 1) {
       dropped = true;
       break;
     }
     age += a.interval;
+    __syncthreads();  // the next sample reads the counters and indices
   }
   __syncthreads();
+  osc_store_indices(a, anl, s_index, tid, blk, n);
   if (!dropped) {
     for (int ai = 0; ai < a.n_analyses; ++ai) {
       const AnalysisDesc& A = a.analyses[ai];
@@ -1849,7 +1961,7 @@ inline int sm_count() {
     cudaLaunchConfig_t cfg{};                                                                   \
     cfg.gridDim = dim3(n_sets * ranks);                                                         \
     cfg.blockDim = dim3(threads);                                                               \
-    cfg.dynamicSmemBytes = a.n_analyses > 0 ? sizeof(double) * a.n_vals * threads : 0;          \
+    cfg.dynamicSmemBytes = a.n_analyses > 0 ? sizeof(double) * a.n_vals * (threads + kValsPad) : 0; \
     cfg.stream = s;                                                                             \
     cfg.attrs = &attr;                                                                          \
     cfg.numAttrs = 1;                                                                           \
