@@ -92,6 +92,7 @@ def lib():
         L.dense_mlp_rank.argtypes = [vp, i, i, vp, vp, i, d, i, vp, vp, i, vp, vp, d, d, d, d, d, vp, vp, vp]
         L.dense_mlp_train_pass.argtypes = [vp, i, i, i, vp, vp, i, vp, i, vp, vp, vp, f, vp, vp, i64, vp, vp]
         L.dense_mlp_train_finish.argtypes = [vp, i64, i, i] + [vp] * 11
+        L.dense_mlp_train_epoch.argtypes = [vp, i, i, i, vp, vp, i, vp, i, i, vp, vp, vp, i64] + [vp] * 9
         _lib = L
     return _lib
 
@@ -253,6 +254,17 @@ class Kernels:
                                              *[_pp(t) for t in state], _p(net._packed if net else None),
                                              self._s()) == 0
 
+    def train_epoch(self, X, T, mask, idx, hyper, loss, work, net):
+        """hyper.shape[0] steps of `net` on the rows that idx gives each, from
+        weights packed for a training pass."""
+        steps = hyper.shape[0]
+        assert hyper.shape[1] == 8 and idx.numel() % steps == 0
+        assert self.L.dense_mlp_train_epoch(_p(X), X.shape[1], X.shape[0], X.shape[1], _p(T), _p(mask), T.shape[1],
+                                            _p(idx), idx.numel() // steps, steps, _p(hyper), _p(loss), _p(work),
+                                            work.numel(), *[_pp(t) for t in (net.W, net.b, net.mW, net.vW, net.mb,
+                                                                             net.vb)],
+                                            _p(net._packed), _p(self.err), self._s()) == 0
+
     def check(self):
         self.torch.cuda.synchronize(self.dev)
         e = int(self.err.item())
@@ -372,36 +384,32 @@ class MLP:
         self.k.check()
         return float(loss.item()), dW, db
 
-    def _train_graphs(self, data, batch, steps):
-        """CUDA graphs of training on the device-resident training set
-        `data` = (X, T, mask), `steps` steps of `batch` rows per epoch.
-        Per epoch the host writes the epoch's row indices ("idx", steps x
+    def _train_buffers(self, batch, steps):
+        """Per epoch the host writes the epoch's row indices ("idx", steps x
         batch) and per-step scalars ("hyper", steps x {lr, b1, b2, eps,
-        1 - b1^t, 1 - b2^t, 1 / count}) into static device buffers.  One
-        process: one graph replays the whole epoch, three launches per step
-        (the batch forward and back, the weight gradients, Adam and the
-        weights' next layout).  Data-parallel: per
-        step a gradient graph and an update graph, with the gradient
-        all-reduce between them.  The graphs hold the addresses of this
-        object's work buffers: they serve one fit call only (no other pass
-        may resize a buffer meanwhile)."""
+        1 - b1^t, 1 - b2^t, 1 / count}) into these device buffers."""
         torch = self.torch
-        g = {}
-        g["idx"] = torch.zeros(steps * batch, dtype=torch.int32, device=self.dev)
-        g["hyper"] = torch.zeros((steps, 8), device=self.dev)
-        g["loss"] = torch.zeros(1, device=self.dev)
+        return {"idx": torch.zeros(steps * batch, dtype=torch.int32, device=self.dev),
+                "hyper": torch.zeros((steps, 8), device=self.dev),
+                "loss": torch.zeros(1, device=self.dev)}
+
+    def _train_graphs(self, g, data, batch, steps):
+        """CUDA graphs of data-parallel training on the device-resident
+        training set `data` = (X, T, mask), `steps` steps of `batch` rows per
+        epoch, reading the buffers g: per step a gradient graph and an update
+        graph, with the gradient all-reduce between them.  The graphs hold
+        the addresses of this object's work buffers: they serve one fit call
+        only (no other pass may resize a buffer meanwhile)."""
+        torch = self.torch
         Xd, Td, Md = data
         work = self._work(batch)
         packed = self._packed
         dW, db = g["dW"], g["db"] = self._grads()
 
-        def pass_(j):
-            self.k.train_pass(Xd, Td, Md, g["idx"][j * batch:(j + 1) * batch], batch, packed, self.b,
-                              g["hyper"][j, 6:7], g["loss"], work)
-
         def grads(j):
             self._pack(backward=True)
-            pass_(j)
+            self.k.train_pass(Xd, Td, Md, g["idx"][j * batch:(j + 1) * batch], batch, packed, self.b,
+                              g["hyper"][j, 6:7], g["loss"], work)
             self.k.train_finish(work, batch, self.n_out, dW, db)
 
         def update(j):
@@ -416,24 +424,15 @@ class MLP:
             grads(0)  # a first launch of each kernel before capture; changes no weight
         torch.cuda.current_stream(self.dev).wait_stream(side)
         torch.cuda.synchronize(self.dev)
-        if self.group is None:
-            g["epoch"] = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g["epoch"]):
-                self._pack(backward=True)
-                for j in range(steps):
-                    pass_(j)
-                    self.k.train_finish(work, batch, self.n_out, hyper=g["hyper"][j], net=self)
-        else:
-            g["grads"], g["update"] = [], []
-            for j in range(steps):
-                gg, gu = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
-                with torch.cuda.graph(gg):
-                    grads(j)
-                with torch.cuda.graph(gu):
-                    update(j)
-                g["grads"].append(gg)
-                g["update"].append(gu)
-        return g
+        g["grads"], g["update"] = [], []
+        for j in range(steps):
+            gg, gu = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+            with torch.cuda.graph(gg):
+                grads(j)
+            with torch.cuda.graph(gu):
+                update(j)
+            g["grads"].append(gg)
+            g["update"].append(gu)
 
     def _fit_epochs(self, X, T, mask, n, epochs, batch, rng, cosine, data=None, b1=0.9, b2=0.999, eps=1e-8):
         """Generator behind the captured fit: each next() enqueues one epoch
@@ -448,7 +447,9 @@ class MLP:
             return
         if data is None:
             data = device_training_set(X, T, mask, self.dev)
-        g = self._train_graphs(data, batch, steps)
+        g = self._train_buffers(batch, steps)
+        if self.group is not None:
+            self._train_graphs(g, data, batch, steps)
         lr0 = self.lr
         total = epochs * steps
         for ep in range(epochs):
@@ -466,7 +467,13 @@ class MLP:
             g["hyper"].copy_(torch.as_tensor(hyp.astype(np.float32)))
             g["loss"].zero_()
             if self.group is None:
-                g["epoch"].replay()
+                # one call launches the epoch's steps, four kernels each: 10 us
+                # a step of the host's time, below the step's on the GPU, so a
+                # graph of them gains nothing and its capture cost more than
+                # a short fit (57 steps: 14.5 ms with one, 11.2 without; four
+                # networks at once over 40 epochs: 203 and 212)
+                self._pack(backward=True)
+                self.k.train_epoch(*data, g["idx"], g["hyper"], g["loss"], self._work(batch), self)
             else:
                 from .distributed import average_
                 for j in range(steps):
@@ -500,9 +507,11 @@ class MLP:
     def fit(self, X, T, mask, epochs=20, batch=4096, seed=0, log=None, cosine=True, captured=True):
         """Minibatch Adam; with `cosine` the learning rate follows a cosine
         from lr down to lr/100 over the run.  With `captured` (the default)
-        the training set is copied to the GPU once and every step replays
-        two CUDA graphs (gradient, update); otherwise each step is launched
-        from the host (`step`), with the same batches and schedule."""
+        the training set is copied to the GPU once and its rows are
+        gathered there (one call launches an epoch; with a group every step
+        replays two CUDA graphs, gradient and update); otherwise each step
+        is launched from the host (`step`), with the same batches and
+        schedule."""
         rng = np.random.Generator(np.random.PCG64(seed))
         n = X.shape[0]
         if self.group is not None:
@@ -546,8 +555,8 @@ def device_training_set(X, T, mask, dev):
 
 def fit_concurrently(nets, X, T, mask, seeds, epochs=20, batch=4096, log=None, cosine=True):
     """MLP.fit of several networks of one process at once, each on its own
-    CUDA stream (a network's epoch is one graph replay; the GEMMs of one
-    4096-row batch fill only a few dozen SMs, so the networks share the
+    CUDA stream (a network's epoch is one call, and the tiles of one
+    4096-row batch fill only a part of the SMs, so the networks share the
     GPU).  Network k takes the batches of seed seeds[k]: its weights are
     those of nets[k].fit(..., seed=seeds[k]).  Returns the loss histories."""
     import torch
@@ -616,8 +625,8 @@ def bench_gemm(rows=131072, reps=20, device=0):
 
 def bench_fit(rows=200000, epochs=3, batch=4096, n_in=44, n_out=5, device=0):
     """Wall time per training step of MLP.fit on seeded random data, the
-    captured form (one CUDA graph per epoch) and the launched form; each
-    after a one-epoch warm-up on a slice, graph capture included."""
+    device-resident form (one call per epoch) and the launched form; each
+    after a one-epoch warm-up on a slice."""
     import time
     import torch
     rng = np.random.Generator(np.random.PCG64(0))

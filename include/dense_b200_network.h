@@ -52,6 +52,15 @@ int dense_mlp_train_finish(const void* work, int64_t work_bytes, int rows, int n
                            float* const* db, const float* hyper, float* const* W, float* const* b, float* const* mW,
                            float* const* vW, float* const* mb, float* const* vb, void* packed, void* stream);
 
+/* `steps` steps of such a pass and finish one after the other: step j takes
+ * the `rows` rows idx[j * rows ..] and the scalars hyper[8 * j ..] ({lr, b1,
+ * b2, eps, 1 - b1^t, 1 - b2^t, inv_count}), both on the device.  `packed`
+ * holds the weights' packing on entry, and that of the new weights after. */
+int dense_mlp_train_epoch(const float* X, int ldx, int x_rows, int n_in, const float* T, const float* mask, int n_out,
+                          const int* idx, int rows, int steps, const float* hyper, float* loss, void* work,
+                          int64_t work_bytes, float* const* W, float* const* b, float* const* mW, float* const* vW,
+                          float* const* mb, float* const* vb, void* packed, int* err, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -13,7 +13,7 @@ def test_declared_symbols_are_exported():
     lib = C.CDLL(surrogate.build())
     text = open(os.path.join(ROOT, "include", "dense_b200_network.h")).read()
     names = set(re.findall(r"^int(?:64_t)? (dense_mlp_[a-z0-9_]+)\(", text, re.M))
-    assert len(names) == 7, names
+    assert len(names) == 8, names
     for name in names:
         assert hasattr(lib, name), name
 
@@ -45,3 +45,7 @@ def test_bad_arguments_are_refused():
     assert L.dense_mlp_train_finish(p, need, 300, 5, None, None, None, *none6, None, None) == 1  # nothing asked for
     assert L.dense_mlp_train_finish(p, need, 300, 5, None, None, p, *none6, p, None) == 1       # Adam without weights
     assert L.dense_mlp_train_finish(p, need - 1, 300, 5, four, four, None, *none6, None, None) == 1
+    epoch = lambda steps, idx, hyper: L.dense_mlp_train_epoch(  # noqa: E731
+        p, 44, 300, 44, p, p, 5, idx, 300, steps, hyper, p, p, need - 1, *[four] * 6, p, p, None)
+    assert epoch(1, p, p) == epoch(-1, p, p) == epoch(0, None, p) == epoch(0, p, None) == 1
+    assert epoch(0, p, p) == 0
