@@ -280,6 +280,7 @@ int build_analyses(const dense_run_desc* run, int num_sets, const dense_set_desc
   int min_cells = kMaxCells + 1;
   for (int s = 0; s < num_sets; ++s) min_cells = std::min(min_cells, in_sets[s].num_cells);
   int64_t anl_block = 0;
+  int queues = 0;
   for (int ai = 0; ai < run->num_analyses; ++ai) {
     const dense_analysis_desc& in = run->analyses[ai];
     AnalysisDesc A{};
@@ -314,6 +315,8 @@ int build_analyses(const dense_run_desc* run, int num_sets, const dense_set_desc
       if (!(rs < 1e6)) return fail(DENSE_ERR_UNSUPPORTED, "oscillation window too long");
       A.range_steps = static_cast<int>(rs);
       A.interval = in.anlys_intvl;
+      A.queue = queues + A.nsp <= kIndexSlots ? queues : -1;
+      if (A.queue >= 0) queues += A.nsp;
       anl_block += 2 + m * A.nsp * kOscFields + static_cast<int64_t>(A.nsp) * (A.range_steps + 1) * m;
     } else if (in.kind == DENSE_ANALYSIS_CONCCHECK) {
       A.lo = in.lower;
@@ -851,7 +854,7 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
   e->analyses.assign(a.analyses, a.analyses + a.n_analyses);
   size_t smem = a.n_analyses > 0 ? sizeof(double) * a.n_vals * (a.block_threads + kValsPad) : 0;
   const size_t csr_bytes = sizeof(int) * max_edges;
-  const size_t smem_cap = a.block_threads <= 224 ? 100000 : 200000;
+  const size_t smem_cap = a.block_threads <= 224 ? kStepSmem2 : kStepSmem1;
   a.csr_in_smem = smem + csr_bytes <= smem_cap ? 1 : 0;
   if (a.csr_in_smem) smem += csr_bytes;
   if (smem > smem_cap) return fail(DENSE_ERR_UNSUPPORTED, "shared memory need of the batch too large");

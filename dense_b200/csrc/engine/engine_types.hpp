@@ -20,6 +20,11 @@ constexpr int kMaxAnalyses = 8;
 constexpr int kStepThreads = 256;  // register kernel: one thread per cell, one CTA per set
 constexpr int kMaxCells = 65536;   // memory kernel: cells per set
 constexpr int kValsPad = 2;        // register kernel: doubles between the rows of the sampled state
+// Register kernel: dynamic shared memory of a CTA, of two and of one per SM
+// (the padding comes on top).
+constexpr int kStepSmem2 = 100000 + 8 * kValsPad * kNS;
+constexpr int kStepSmem1 = 200000 + 8 * kValsPad * kNS;
+constexpr int kIndexSlots = 64;    // queue indices of oscillation analyses that a CTA shares
 constexpr int kMaxCluster = 16;    // register kernel: CTAs a set's cells may be spread over (above the portable 8)
 constexpr int kClusterSmem = 100000;  // dynamic shared memory of such a CTA (two per SM)
 constexpr int64_t kMaxRegisterRing = 1 << 25;  // register kernel: elements of one set's history rings
@@ -48,6 +53,7 @@ struct AnalysisDesc {
   double interval;      // oscillation anlys-intvl
   double lo, hi;        // concentration check bounds
   int64_t off;          // offset of this analysis' state inside a set's block
+  int queue;            // oscillation: first of its species' queue indices in the CTA's copy, -1: each cell's own
 };
 
 // Layout of one analysis' per-set state (doubles), relative to
@@ -103,7 +109,9 @@ struct SetDesc {
 // Dynamic shared memory a wave-kernel CTA may use (the 227 KB opt-in limit
 // of sm_100 less room for the kernel's static shared memory), and the
 // neighbours a wave-kernel cell record holds.
-constexpr int kWaveSmemBudget = 227 * 1024 - 8 * 1024;
+constexpr int kWaveStatic = 8 * kNP + 8 * kND * kNS + 40 * kNS + 16 * kIndexSlots + 512;
+constexpr int kWaveRoom = kWaveStatic > 8 * 1024 ? (kWaveStatic + 1023) / 1024 * 1024 : 8 * 1024;
+constexpr int kWaveSmemBudget = 227 * 1024 - kWaveRoom;
 constexpr int kWaveMaxNbrs = 6;
 constexpr int kWaveMaxFronts = 4;   // steps in flight in the wave kernel
 

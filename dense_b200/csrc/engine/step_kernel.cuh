@@ -215,7 +215,7 @@ enum ReadMode : int {
 // use.  Measured on a 14-species gene network with 10 own and 2 neighbour
 // reads per cell-step: 1551 instructions per warp-step, 630 of them in the
 // own reads, 2.3 cycles per instruction waiting for loads; now 968 and 1.1
-// (4096 sets x 200 cells x 300 steps with Oscillation: 30.9 -> 16.6 ms a
+// (4096 sets x 200 cells x 300 steps with Oscillation: 30.9 -> 17.5 ms a
 // run; a batch in FP32: 12.1 -> 7.1 ms; one set of 200 perturbed cells x
 // 1000 steps, whole call: 7.9 -> 5.6 ms).  To that end
 //  * everything that does not change from step to step is resolved before
@@ -359,7 +359,7 @@ struct RegContext {
 // The tables of RegContext fit in static shared memory up to this many
 // (delay reaction, species) pairs; models above it form their rows per read.
 constexpr int kPairs = kND * kNS;
-constexpr bool kRowTables = kPairs > 0 && kPairs <= 1024;
+constexpr bool kRowTables = kPairs > 0 && kPairs <= 384;  // 64 bytes a pair
 
 // ------------------------------------------------------------ analyses
 // All per-cell analysis state is structure-of-arrays over the analysed
@@ -491,7 +491,8 @@ __device__ __forceinline__ void osc_add_crit(const OscRef& o, double t, double c
 // samples alone, so every cell of a species has the same: during a launch
 // each CTA keeps one copy per (analysis, species) in shared memory, and the
 // cells' own fields are read when it begins and written when it ends
-// (osc_load_indices, osc_store_indices).  With eight index fields read and
+// (osc_load_indices, osc_store_indices); analyses past kIndexSlots species
+// in all (AnalysisDesc::queue < 0) read and write the fields at each sample.  With eight index fields read and
 // written per cell, species and sample, 100 samples of two species in 160
 // cells took 0.37 ms beside 1000 steps' 2.4 ms, and 0.33 ms so; over 1024
 // sets on a full GPU 1.24 and 1.04 ms.
@@ -621,7 +622,10 @@ __device__ __forceinline__ void osc_cell_update(double* st, const AnalysisDesc& 
     double* win = osc_window(st, A, i, cc);
     const double added = vals(A.slot[i], c);
     OscQueue q;
-    static_cast<OscIndex&>(q) = index[i];
+    if (A.queue >= 0)
+      static_cast<OscIndex&>(q) = index[A.queue + i];
+    else
+      q.load(o);
     // the run of equal newest values (NaN equals nothing)
     const double run = o.f(kOscSame);
     const double newest = q.live > 0 ? win[static_cast<size_t>(q.end) * m] : added;
@@ -630,6 +634,7 @@ __device__ __forceinline__ void osc_cell_update(double* st, const AnalysisDesc& 
     const bool stop = q.sample(w);
     win[static_cast<size_t>(q.end) * m] = added;
     o.f(kOscSame) = static_cast<double>(q.same);
+    if (A.queue < 0) q.store(o);
     if (!stop) osc_check(o, q, win, m, w, samples, A);
     if (stop) break;
   }
@@ -637,33 +642,35 @@ __device__ __forceinline__ void osc_cell_update(double* st, const AnalysisDesc& 
 
 // One thread per analysis: its species' indices past a sample.
 __device__ __forceinline__ void osc_advance(const AnalysisDesc& A, OscIndex* index) {
+  if (A.queue < 0) return;
   for (int i = 0; i < A.nsp; ++i)
-    if (index[i].sample(A.range_steps + 1)) break;
+    if (index[A.queue + i].sample(A.range_steps + 1)) break;
 }
 
 // The indices of every oscillation analysis, from (to) the fields of its
 // first (of every) cell.
-__device__ __forceinline__ void osc_load_indices(const StepArgs& a, double* anl, OscIndex (*index)[kNS], int tid,
+__device__ __forceinline__ void osc_load_indices(const StepArgs& a, double* anl, OscIndex* index, int tid,
                                                  int threads) {
-  for (int k = tid; k < a.n_analyses * kNS; k += threads) {
-    const AnalysisDesc& A = a.analyses[k / kNS];
-    const int i = k % kNS;
-    if (A.kind != kOscillation || i >= A.nsp || A.cmax <= A.cmin) continue;
-    OscQueue q;
-    q.load(osc_ref(anl + A.off, A, i, 0));
-    index[k / kNS][i] = q;
+  for (int ai = 0; ai < a.n_analyses; ++ai) {
+    const AnalysisDesc& A = a.analyses[ai];
+    if (A.kind != kOscillation || A.queue < 0 || A.cmax <= A.cmin) continue;
+    for (int i = tid; i < A.nsp; i += threads) {
+      OscQueue q;
+      q.load(osc_ref(anl + A.off, A, i, 0));
+      index[A.queue + i] = q;
+    }
   }
 }
-__device__ __forceinline__ void osc_store_indices(const StepArgs& a, double* anl, const OscIndex (*index)[kNS], int c0,
+__device__ __forceinline__ void osc_store_indices(const StepArgs& a, double* anl, const OscIndex* index, int c0,
                                                   int stride, int n) {
   for (int ai = 0; ai < a.n_analyses; ++ai) {
     const AnalysisDesc& A = a.analyses[ai];
-    if (A.kind != kOscillation) continue;
+    if (A.kind != kOscillation || A.queue < 0) continue;
     for (int c = c0; c < n; c += stride) {
       if (c < A.cmin || c >= A.cmax) continue;
       for (int i = 0; i < A.nsp; ++i) {
         OscQueue q;
-        static_cast<OscIndex&>(q) = index[ai][i];
+        static_cast<OscIndex&>(q) = index[A.queue + i];
         q.store(osc_ref(anl + A.off, A, i, c - A.cmin));
       }
     }
@@ -722,8 +729,11 @@ struct ClusterVals {
 };
 
 // All threads of the cluster; what they wrote before is visible after.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  cluster_arrive();
+  cluster_wait();
 }
 
 template <typename T>
@@ -747,7 +757,7 @@ struct RingVals {
 template <int kAhead, typename Vals, typename Fold>
 __device__ __forceinline__ bool analyses_sample(const StepArgs& a, double* anl, const Vals& vals, const Fold& fold,
                                                 bool lead, int tid, int c0, int stride, int n, double age,
-                                                const double* samples, const OscIndex (*index)[kNS]) {
+                                                const double* samples, const OscIndex* index) {
   bool bad = false;
   for (int ai = 0; ai < a.n_analyses; ++ai) {
     const AnalysisDesc& A = a.analyses[ai];
@@ -762,7 +772,7 @@ __device__ __forceinline__ bool analyses_sample(const StepArgs& a, double* anl, 
     } else if (A.kind == kOscillation) {
       if (lead && tid == 0) st[1] = age;
       if (!in_range) continue;
-      for (int c = c0; c < n; c += stride) osc_cell_update(st, A, vals, c, samples[ai], index[ai]);
+      for (int c = c0; c < n; c += stride) osc_cell_update(st, A, vals, c, samples[ai], index);
       if (lead && tid == 0) st[0] = samples[ai] + 1.0;
     } else if (A.kind == kTrajectory) {
       // csvw_sim::update (io/csvw_sim.ipp:17-91): every observed species
@@ -832,13 +842,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
   __shared__ __align__(16) T s_prm[kNP];
   __shared__ int s_flags;
   __shared__ double s_samples[kMaxAnalyses];
-  __shared__ OscIndex s_index[kMaxAnalyses][kNS];
-  // resolved reads (own, then neighbour); kTable: their row offsets of this
-  // step and the next, then the rows written, and the entries that advance
+  __shared__ OscIndex s_index[kIndexSlots];
+  // resolved reads (own, then neighbour); kTable: their row offsets, then
+  // the rows written, of this step and the next two, and the entries that
+  // advance
   constexpr int kReads = kUniform ? 2 * kPairs : 0;
   constexpr int kEntries = kTable ? 2 * kPairs + kNS : 0;
   __shared__ int s_res[kReads > 0 ? kReads : 1];
-  __shared__ int s_at[2][kEntries > 0 ? kEntries : 1];
+  __shared__ int s_at[3][kEntries > 0 ? kEntries : 1];
   __shared__ int4 s_live[kEntries > 0 ? kEntries : 1];  // {lag (-1: the row written), depth - 1, ring offset, entry}
   __shared__ int s_n_live;
 
@@ -898,8 +909,23 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
       }
     }
   }
-  if (kTable) {
+  // Rows of lag 1 and more are published a barrier before the one that ends
+  // the step they are read after: unless a neighbour's row of lag 0 is read,
+  // a step's loads go out before that barrier, under the wait for the others
+  // (kernel times behind it and before it: 4096 sets x 200 cells x 300 steps
+  // 13.5 and 12.9 ms, 2000 sets in FP32 5.73 and 5.37, 96 sets x 733 cells x
+  // 200 steps on clusters 1.81 and 1.69, one set of 200 cells x 1000 steps
+  // 3.61 and 3.47).
+  bool reads_lag0 = false;
+  if (kUniform) {
     __syncthreads();
+    for (int i = c; i < kPairs; i += blk) reads_lag0 = reads_lag0 || s_res[kPairs + i] == 0;
+  } else {
+#pragma unroll
+    for (int i = 0; i < kPairs; ++i) reads_lag0 = reads_lag0 || lres[kPairs + i] == 0;
+  }
+  const bool loads_early = __syncthreads_or(reads_lag0) == 0;
+  if (kTable) {
     for (int e = c; e < kEntries; e += blk) {
       int at = -1;
       bool live;
@@ -916,8 +942,11 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
         const int lag = write ? -1 : s_res[e];
         s_live[atomicAdd(&s_n_live, 1)] = make_int4(lag, r.x, r.y, e);
         at = ((static_cast<int>(step) - lag) & r.x) * n + r.y;
+        s_at[1][e] = ((static_cast<int>(step) + 1 - lag) & r.x) * n + r.y;
+      } else {
+        s_at[1][e] = s_at[2][e] = at;
       }
-      s_at[0][e] = s_at[1][e] = at;
+      s_at[0][e] = at;
     }
   }
 
@@ -969,6 +998,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
       checks = checks || a.analyses[i].kind == kConcCheck;
     }
 
+  int table_now = 0;  // of the row tables
   for (; chunk < chunk_end; ++chunk) {
     // ---- analyses sample the state at `age` (measurement/base.ipp:4-9)
     if (a.n_analyses > 0) {
@@ -1003,7 +1033,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
       // queue indices
       if (c < a.n_analyses && !(age < a.analyses[c].t0 || age >= a.analyses[c].t1)) {
         s_samples[c] += 1.0;
-        if (a.analyses[c].kind == kOscillation) osc_advance(a.analyses[c], s_index[c]);
+        if (a.analyses[c].kind == kOscillation) osc_advance(a.analyses[c], s_index);
       }
       int flags = s_flags;
       if (kCluster && checks)
@@ -1017,56 +1047,74 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
     // ---- (int)(interval/dt) Euler steps (determ.cpp:8-21, 77-88)
     for (int s = 0; s < steps_per_chunk; ++s) {
       T nxt[kNS];
-      const int* at = s_at[ctx.step & 1];
+      const int* at = s_at[table_now];
       if (kTable) {
         ctx.own_at = at;
         ctx.nbr_at = at + kPairs;
-        // the next step's rows
-        int* next = s_at[(ctx.step + 1) & 1];
-        for (int i = c; i < n_live; i += blk) {
-          const int4 e = s_live[i];
-          next[e.w] = ((ctx.step + 1 - e.x) & e.y) * n + e.z;
-        }
       }
-      if (active) {
-        // DENSE evaluates every rate, then adds rate * delta reaction by
-        // reaction (determ.cpp:58-72).  Each species' accumulator sees the
-        // same additions in the same order when each rate is folded in as
-        // soon as it is known, which keeps one rate live instead of all.
-        T dsp[kNS];
+      // the barrier that ends the step before, around this step's loads
+      // (threads without a cell go along with cell 0 and write nothing)
+      if (kCluster) {
+        cluster_arrive();
+        if (!loads_early) cluster_wait();
+      } else if (!loads_early) {
+        __syncthreads();
+      }
+      fetched.seen = 0;
 #pragma unroll
-        for (int sp = 0; sp < kNS; ++sp) dsp[sp] = T(0);
-        fetched.seen = 0;
-#pragma unroll
-        for (int i = 0; i < kPairs; ++i) fetched.has_own[i] = fetched.has_nbr[i] = false;
+      for (int i = 0; i < kPairs; ++i) fetched.has_own[i] = fetched.has_nbr[i] = false;
 #define REACTION(name) (void)reaction<name>::active_rate(ctx);
 #include "reactions_list.hpp"
 #undef REACTION
+      if (loads_early) {
+        if (kCluster) {
+          cluster_wait();
+        } else {
+          __syncthreads();
+        }
+      }
+      if (kTable) {
+        // the rows of the step after the next
+        table_now = table_now == 2 ? 0 : table_now + 1;
+        int* then = s_at[table_now == 2 ? 0 : table_now + 1];
+        for (int i = c; i < n_live; i += blk) {
+          const int4 e = s_live[i];
+          then[e.w] = ((ctx.step + 2 - e.x) & e.y) * n + e.z;
+        }
+      }
+      // DENSE evaluates every rate, then adds rate * delta reaction by
+      // reaction (determ.cpp:58-72).  Each species' accumulator sees the
+      // same additions in the same order when each rate is folded in as
+      // soon as it is known, which keeps one rate live instead of all.
+      T dsp[kNS];
+#pragma unroll
+      for (int sp = 0; sp < kNS; ++sp) dsp[sp] = T(0);
 #define REACTION(name)                                                        \
   {                                                                           \
     const T rate_ = reaction<name>::active_rate(rctx);                        \
     _Pragma("unroll") for (int j = 0; j < num_deltas_##name; j++)             \
         dsp[delta_ids_##name[j]] += rate_ * static_cast<T>(deltas_##name[j]); \
   }
-        if (__builtin_expect((fetched.seen & kReadCheckBit) == 0, 1)) {
-          const auto rctx = ctx.template as<kUse>();
+      if (__builtin_expect((fetched.seen & kReadCheckBit) == 0, 1)) {
+        const auto rctx = ctx.template as<kUse>();
 #include "reactions_list.hpp"
-        } else {
-          const auto rctx = ctx.template as<kChecked>();
+      } else {
+        const auto rctx = ctx.template as<kChecked>();
 #include "reactions_list.hpp"
-        }
+      }
 #undef REACTION
 #pragma unroll
-        for (int sp = 0; sp < kNS; ++sp) {
-          if (kKahan) {
-            const T y = dt * dsp[sp] - comp[sp];
-            const T t = cur[sp] + y;
-            comp[sp] = (t - cur[sp]) - y;
-            nxt[sp] = t;
-          } else {
-            nxt[sp] = cur[sp] + dt * dsp[sp];
-          }
+      for (int sp = 0; sp < kNS; ++sp) {
+        if (kKahan) {
+          const T y = dt * dsp[sp] - comp[sp];
+          const T t = cur[sp] + y;
+          comp[sp] = (t - cur[sp]) - y;
+          nxt[sp] = t;
+        } else {
+          nxt[sp] = cur[sp] + dt * dsp[sp];
         }
+      }
+      if (active) {
 #pragma unroll
         for (int sp = 0; sp < kNS; ++sp) {
           if (kTable) {
@@ -1078,16 +1126,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
           }
         }
       }
-      if (kCluster) {
-        cluster_barrier();
-      } else {
-        __syncthreads();
-      }
       ctx.step += 1;
-      if (active) {
 #pragma unroll
-        for (int sp = 0; sp < kNS; ++sp) cur[sp] = nxt[sp];
-      }
+      for (int sp = 0; sp < kNS; ++sp) cur[sp] = nxt[sp];
     }
     step += steps_per_chunk;
     age += a.interval;
@@ -1176,7 +1217,7 @@ __global__ void __launch_bounds__(256, 2) dense_step_mem_kernel(const StepArgs a
   __shared__ T s_prm[kNP];
   __shared__ int s_flags;
   __shared__ double s_samples[kMaxAnalyses];
-  __shared__ OscIndex s_index[kMaxAnalyses][kNS];
+  __shared__ OscIndex s_index[kIndexSlots];
   __shared__ int s_olag[kND > 0 ? kND * kNS : 1], s_nlag[kND > 0 ? kND * kNS : 1];
   __shared__ T* s_rows[kNS];
   __shared__ T* s_crows[kNS];
@@ -1242,7 +1283,7 @@ __global__ void __launch_bounds__(256, 2) dense_step_mem_kernel(const StepArgs a
       if (tid < a.n_analyses) {
         const AnalysisDesc& A = a.analyses[tid];
         s_samples[tid] = anl[A.off];
-        if (A.kind == kOscillation && !(age < A.t0 || age >= A.t1)) osc_advance(A, s_index[tid]);
+        if (A.kind == kOscillation && !(age < A.t0 || age >= A.t1)) osc_advance(A, s_index);
       }
       if (s_flags & 1) {
         dropped = true;
@@ -1474,7 +1515,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_wave_kernel(c
   __shared__ T s_prm[kNP];
   __shared__ int s_flags;
   __shared__ double s_samples[kMaxAnalyses];
-  __shared__ OscIndex s_index[kMaxAnalyses][kNS];
+  __shared__ OscIndex s_index[kIndexSlots];
   __shared__ int s_olag[kND > 0 ? kND * kNS : 1], s_nlag[kND > 0 ? kND * kNS : 1];
   __shared__ T* s_rows[kNS];
   __shared__ T* s_crows[kNS];
@@ -1605,7 +1646,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_wave_kernel(c
       if (tid < a.n_analyses) {
         const AnalysisDesc& A = a.analyses[tid];
         s_samples[tid] = anl[A.off];
-        if (A.kind == kOscillation && !(age < A.t0 || age >= A.t1)) osc_advance(A, s_index[tid]);
+        if (A.kind == kOscillation && !(age < A.t0 || age >= A.t1)) osc_advance(A, s_index);
       }
       if (s_flags & 1) {
         dropped = true;
@@ -1755,7 +1796,7 @@ template <typename T>
 __global__ void dense_import_kernel(const StepArgs a, int set, const double* samples, int num_samples,
                                     double time_start) {
   __shared__ double s_samples[kMaxAnalyses];
-  __shared__ OscIndex s_index[kMaxAnalyses][kNS];
+  __shared__ OscIndex s_index[kIndexSlots];
   __shared__ int s_flags;
   const SetDesc& sd = a.sets[set];
   const int n = sd.n_cells;
@@ -1776,7 +1817,7 @@ __global__ void dense_import_kernel(const StepArgs a, int set, const double* sam
     if (tid < a.n_analyses) {
       const AnalysisDesc& A = a.analyses[tid];
       s_samples[tid] = anl[A.off];
-      if (A.kind == kOscillation && !(age < A.t0 || age >= A.t1)) osc_advance(A, s_index[tid]);
+      if (A.kind == kOscillation && !(age < A.t0 || age >= A.t1)) osc_advance(A, s_index);
     }
     if (s_flags & 1) {
       dropped = true;
@@ -1980,11 +2021,11 @@ inline int sm_count() {
     /* two 224-thread CTAs per SM (128 registers) when the sets fill more  \
        than one CTA per SM; else one CTA per SM with every register */     \
     if (a.block_threads <= 224 && n_sets > sm_count()) {                                        \
-      if (a.uniform_params) DENSE_B200_STEP_VARIANT(T, KAHAN, 224, 2, true, 100000)              \
-      else DENSE_B200_STEP_VARIANT(T, KAHAN, 224, 2, false, 100000)                               \
+      if (a.uniform_params) DENSE_B200_STEP_VARIANT(T, KAHAN, 224, 2, true, kStepSmem2)              \
+      else DENSE_B200_STEP_VARIANT(T, KAHAN, 224, 2, false, kStepSmem2)                               \
     } else {                                                                                    \
-      if (a.uniform_params) DENSE_B200_STEP_VARIANT(T, KAHAN, 256, 1, true, 200000)              \
-      else DENSE_B200_STEP_VARIANT(T, KAHAN, 256, 1, false, 200000)                               \
+      if (a.uniform_params) DENSE_B200_STEP_VARIANT(T, KAHAN, 256, 1, true, kStepSmem1)              \
+      else DENSE_B200_STEP_VARIANT(T, KAHAN, 256, 1, false, kStepSmem1)                               \
     }                                                                                           \
   }                                                                                             \
   }

@@ -58,3 +58,15 @@ def test_wave_kernel(chunks):
     sets = _grid(100, 10, 3, duration=2.0)
     N.assert_same(N.oracle_states(N.GRID, sets, 0.01, 0.1, an),
                   N.engine_states(N.GRID, sets, 0.01, 0.1, an, chunks=chunks))
+
+
+def test_more_analyses_than_shared_indices():
+    """Seven equal analyses of thirteen species: the fields of the last ones
+    are read and written at each sample."""
+    from dense_b200 import engine as E
+    an = [E.Analysis.oscillation(list(range(13)), 0, 50, 0.0, float("inf"), 0.4, 0.1) for _ in range(7)]
+    sets = _sets(50, False, 12, count=2, duration=2.0)
+    got = N.engine_states(N.NETWORK, sets, 0.01, 0.1, an, chunks=6)
+    for g in got:
+        for k in range(1, 7):
+            N.assert_same([{"": g[0]}], [{"": g[k]}])
