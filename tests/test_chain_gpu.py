@@ -159,3 +159,23 @@ def test_empty_inputs_and_refusals():
     assert net.predict(np.zeros((0, 44), np.float32)).shape == (0, 5)
     with pytest.raises(RuntimeError):
         net.predict_device(torch.zeros((3, 43), device="cuda"))
+
+
+@pytest.mark.parametrize("n_out", [5, 64, 65, 128])
+@pytest.mark.parametrize("rows", [4097, 4224, 4225, 4353, 5000])
+def test_gradients_around_the_last_cluster(rows, n_out):
+    """One cluster of CTAs a tile up to as many as the GPU holds, one CTA a
+    tile above: bias gradients bit for bit, weight gradients as sums of the
+    same products in another order (float32, 1e-5)."""
+    import torch
+    net = _net(44, n_out, 1)
+    rng = np.random.Generator(np.random.PCG64(rows))
+    X = rng.uniform(-1, 1, size=(rows, 44)).astype(np.float32)
+    T = rng.normal(size=(rows, n_out)).astype(np.float32)
+    mask = (rng.uniform(size=T.shape) > 0.3).astype(np.float32)
+    loss, dW, db = _layered(net, *(torch.tensor(v, device="cuda") for v in (X, T, mask)))
+    got, gW, gb = net.gradients(X, T, mask)
+    assert abs(got - loss) <= 1e-5 * abs(loss)
+    for i in range(4):
+        assert torch.equal(gb[i], db[i])
+        assert (gW[i] - dW[i]).norm() <= 1e-5 * dW[i].norm()
