@@ -179,3 +179,41 @@ def test_gradients_around_the_last_cluster(rows, n_out):
     for i in range(4):
         assert torch.equal(gb[i], db[i])
         assert (gW[i] - dW[i]).norm() <= 1e-5 * dW[i].norm()
+
+
+@pytest.mark.parametrize("rows", [300, 6000])
+def test_steps_in_a_captured_graph(rows):
+    """Pass and finish of two steps, replayed: the weights of the same steps
+    launched one by one."""
+    import torch
+    rng = np.random.Generator(np.random.PCG64(rows))
+    f = lambda x: torch.tensor(x.astype(np.float32), device="cuda")  # noqa: E731
+    X, T = f(rng.uniform(-1, 1, size=(rows, 44))), f(rng.normal(size=(rows, 5)))
+    mask = torch.ones_like(T)
+    hyper = f(np.array([[1e-3, 0.9, 0.999, 1e-8, 1 - 0.9 ** t, 1 - 0.999 ** t, 1.0 / rows, 0.0] for t in (1, 2)]))
+    got = []
+    for graph in (False, True):
+        net = _net(44, 5, 3)
+        work, loss = net._work(rows), torch.zeros(1, device="cuda")
+        idx = torch.arange(rows, dtype=torch.int32, device="cuda").repeat(2)
+        net._pack(backward=True)
+        run = lambda: net.k.train_epoch(X, T, mask, idx, hyper, loss, work, net)  # noqa: E731
+        if graph:
+            held = [t.clone() for t in net.W + net.b]
+            run()  # a first launch of each kernel
+            for t, h in zip(net.W + net.b, held):
+                t.copy_(h)
+            for t in net.mW + net.vW + net.mb + net.vb:
+                t.zero_()
+            net._pack(backward=True)
+            torch.cuda.synchronize()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                run()
+            g.replay()
+        else:
+            run()
+        net.k.check()
+        got.append([t.clone() for t in net.W + net.b])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
