@@ -883,7 +883,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
   double* anl = a.anl + sd.anl_base;
   if (c < a.n_analyses) s_samples[c] = anl[a.analyses[c].off];
   osc_load_indices(a, anl, s_index, c, blk);
-  __syncthreads();
+  if (kCluster && a.n_analyses > 0) {
+    // rank 0 advances the counters in the set's block at the first sample:
+    // every CTA has its copy before (the CTAs of a cluster run at the same
+    // time, but start at their own)
+    cluster_barrier();
+  } else {
+    __syncthreads();
+  }
 
   const int cell = active ? first + c : 0;
   // parameters: the shared row of the set, or this cell's column of the
