@@ -1016,7 +1016,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_kernel(const 
         s_vals[row * (blk + kValsPad) + c] =
             static_cast<double>(cur[sp]) - (kKahan ? static_cast<double>(comp[sp]) : 0.0);
       }
-      if (kCluster && folds) {
+      // (without steps in between, the flags of the chunk before have been
+      // read in every CTA before a sample sets them again)
+      if (kCluster && (folds || (checks && steps_per_chunk == 0))) {
         cluster_barrier();
       } else {
         __syncthreads();
