@@ -147,7 +147,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 // kernels before to be complete and their writes visible; nothing of theirs
 // is read, or written over, before.  Then lets the next one start.  (Every
 // kernel of the sequence waits, so that each also follows the ones before
-// the one before.)  2048 rows, pass, bias sums and weight gradients: 49 us
+// the one before.)  A kernel that calls this is resident while the one before
+// still writes what it reads, so its global loads are plain ones through
+// unqualified pointers: __restrict__ and the read-only and cache-hinted load
+// functions let the compiler take the memory for constant and move a load
+// above the wait.  2048 rows, pass, bias sums and weight gradients: 49 us
 // one after the other, 43 so.
 __device__ __forceinline__ void follow_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -522,7 +526,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const __gri
             tmem_ld16(acc + col, v);
 #pragma unroll
             for (int j = 0; j < 16; j += 4) {
-              const float4 b = __ldg(reinterpret_cast<const float4*>(bias + col + j));
+              const float4 b = *reinterpret_cast<const float4*>(bias + col + j);
               v[j] += b.x;
               v[j + 1] += b.y;
               v[j + 2] += b.z;
@@ -925,7 +929,7 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kChainThreads, 
       tmem_ld16(lanes + (layer & 1) * 128 + g * 16, v);
 #pragma unroll
       for (int j = 0; j < 16; j += 4) {
-        const float4 b = __ldg(reinterpret_cast<const float4*>(bias + j));
+        const float4 b = *reinterpret_cast<const float4*>(bias + j);
         v[j] += b.x;
         v[j + 1] += b.y;
         v[j + 2] += b.z;
@@ -1153,8 +1157,8 @@ __global__ void __launch_bounds__(kWgradThreads, 1) mlp_wgrad_kernel(const Wgrad
 // Block (column group of 32, slice).
 constexpr int kColSlices = 8;
 
-__global__ void __launch_bounds__(256) mlp_bias_sums_kernel(const float* __restrict__ dz, const float* __restrict__ dy,
-                                                            int tiles, int oc, float* __restrict__ db_part) {
+__global__ void __launch_bounds__(256) mlp_bias_sums_kernel(const float* dz, const float* dy, int tiles, int oc,
+                                                            float* db_part) {
   __shared__ float part[32][33];
   follow_previous();
   const int y = threadIdx.x & 31, w = threadIdx.x >> 5;  // row lane, four columns
@@ -1237,9 +1241,9 @@ __global__ void __launch_bounds__(256) mlp_finish_kernel(const __grid_constant__
     int at;
     const int layer = layer_of(t * 4, &at);
     const float4* p = reinterpret_cast<const float4*>(a.parts) + t;
-    float4 s = __ldcs(p);
+    float4 s = *p;
     for (int k = 1; k < a.splits; ++k) {
-      const float4 x = __ldcs(p + static_cast<int64_t>(k) * (kWeights / 4));
+      const float4 x = p[static_cast<int64_t>(k) * (kWeights / 4)];
       s.x += x.x;
       s.y += x.y;
       s.z += x.z;
