@@ -28,6 +28,7 @@
 
 #include "count_div.cuh"
 #include "engine_types.hpp"
+#include "per_device.hpp"
 
 namespace dense_b200 {
 
@@ -1916,43 +1917,54 @@ __global__ void dense_init_kernel(const StepArgs a, const double* init_conc, con
   }
 }
 
-}  // namespace dense_b200
-
-// Streaming multiprocessors of the current device (looked up once).
+// Streaming multiprocessors of the current device.
 inline int sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
-      n = v;
-  }
-  return n > 0 ? n : 148;
+  static PerDevice known;
+  static int counts[64] = {};
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+  if (dev < 0 || dev >= 64)
+    return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? n : 148;
+  const cudaError_t e =
+      known.once(dev, [&] { return cudaDeviceGetAttribute(&counts[dev], cudaDevAttrMultiProcessorCount, dev); });
+  return e == cudaSuccess ? counts[dev] : 148;
 }
+
+// A kernel's opt-in to `smem` bytes of dynamic shared memory (and to
+// clusters of more than eight CTAs) on the current device: attributes belong
+// to a device, so each one a process uses is set up (inside no capture after
+// the first launch there).
+template <auto kernel>
+cudaError_t opt_in(int smem, bool large_clusters) {
+  static PerDevice devices;
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  return devices.once(dev, [&] {
+    cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (r == cudaSuccess && large_clusters)
+      r = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return r;
+  });
+}
+
+}  // namespace dense_b200
 
 // Launchers, named by the including translation unit's precision suffix.
 #define DENSE_B200_STEP_VARIANT(T, KAHAN, THREADS, BLOCKS, UNIFORM, SMEM_CAP)                     \
   {                                                                                             \
-    auto k = dense_step_kernel<T, KAHAN, THREADS, BLOCKS, UNIFORM, false>;                      \
-    static bool configured = false;                                                             \
-    if (!configured) {                                                                          \
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_CAP); \
-      if (e != cudaSuccess) return e;                                                           \
-      configured = true;                                                                        \
-    }                                                                                           \
+    constexpr auto k = dense_step_kernel<T, KAHAN, THREADS, BLOCKS, UNIFORM, false>;            \
+    const cudaError_t e = opt_in<k>(SMEM_CAP, false);                                           \
+    if (e != cudaSuccess) return e;                                                             \
     k<<<n_sets, a.block_threads, smem, s>>>(a, set_list);                                       \
     return cudaGetLastError();                                                                  \
   }
 
 #define DENSE_B200_CLUSTER_VARIANT(T, KAHAN, BLOCKS, UNIFORM)                                    \
   {                                                                                             \
-    auto k = dense_step_kernel<T, KAHAN, 256, BLOCKS, UNIFORM, true>;                            \
-    static bool configured = false;                                                             \
-    if (!configured) {                                                                          \
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmem); \
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); \
-      if (e != cudaSuccess) return e;                                                           \
-      configured = true;                                                                        \
-    }                                                                                           \
+    constexpr auto k = dense_step_kernel<T, KAHAN, 256, BLOCKS, UNIFORM, true>;                 \
+    const cudaError_t e = opt_in<k>(kClusterSmem, true);                                        \
+    if (e != cudaSuccess) return e;                                                             \
     return cudaLaunchKernelEx(&cfg, k, a, set_list);                                            \
   }
 
