@@ -630,7 +630,12 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
     SetPlan plan;
     int rc = plan_set(in, dt, run->precision == DENSE_FP64 ? 8 : 4, plan, cp);
     if (rc != DENSE_OK) return fail(rc, where + g_error);
-    if (sample_bytes > kClusterSmem) plan.ranks = 0;
+    // (a device that holds no cluster of that size, or shared memory that a
+    // CTA of one has not got: the memory kernel)
+    if (plan.ranks > 0 && (sample_bytes > kClusterSmem ||
+                           !(run->precision == DENSE_FP64 ? step_cluster_fits_fp64(plan.ranks)
+                                                          : step_cluster_fits_fp32(plan.ranks))))
+      plan.ranks = 0;
     SetDesc& d = plan.d;
     const double chunks = in.duration / interval;  // run_simulation.hpp:127
     if (!(chunks < 2147483647.0)) return fail(DENSE_ERR_INVALID, where + "too many chunks");

@@ -1948,6 +1948,43 @@ cudaError_t opt_in(int smem, bool large_clusters) {
   });
 }
 
+// Clusters of `ranks` CTAs of a kernel, at their largest (256 threads,
+// kClusterSmem bytes), that the current device holds at once; 0 where it
+// cannot run one.
+template <auto kernel>
+int clusters_at_once(int ranks) {
+  if (opt_in<kernel>(kClusterSmem, true) != cudaSuccess) return 0;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = ranks;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ranks);
+  cfg.blockDim = dim3(kStepThreads);
+  cfg.dynamicSmemBytes = kClusterSmem;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  return cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess ? n : 0;
+}
+
+// Whether the current device runs clusters of `ranks` CTAs in every variant
+// of the register kernel a launch may take; asked once per device and size.
+template <typename T, bool kKahan>
+bool cluster_fits(int ranks) {
+  static PerDevice asked[kMaxCluster + 1];
+  int dev = 0;
+  if (ranks < 1 || ranks > kMaxCluster || cudaGetDevice(&dev) != cudaSuccess) return false;
+  const bool missing = asked[ranks].once(dev, [&] {
+    return !(clusters_at_once<dense_step_kernel<T, kKahan, 256, 1, true, true>>(ranks) > 0 &&
+             clusters_at_once<dense_step_kernel<T, kKahan, 256, 1, false, true>>(ranks) > 0 &&
+             clusters_at_once<dense_step_kernel<T, kKahan, 256, 2, true, true>>(ranks) > 0 &&
+             clusters_at_once<dense_step_kernel<T, kKahan, 256, 2, false, true>>(ranks) > 0);
+  });
+  if (missing) cudaGetLastError();
+  return !missing;
+}
+
 }  // namespace dense_b200
 
 // Launchers, named by the including translation unit's precision suffix.
@@ -2013,6 +2050,7 @@ cudaError_t opt_in(int smem, bool large_clusters) {
     }                                                                                           \
     return cudaGetLastError();                                                                  \
   }                                                                                             \
+  bool step_cluster_fits_##SUFFIX(int ranks) { return cluster_fits<T, KAHAN>(ranks); }           \
   cudaError_t launch_step_cluster_##SUFFIX(const StepArgs& a, const int* set_list, int n_sets, int threads, \
                                            int ranks, cudaStream_t s) {                          \
     if (n_sets <= 0) return cudaSuccess;                                                        \
