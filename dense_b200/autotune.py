@@ -2,7 +2,8 @@
 
 A set's results do not depend on how it is scheduled, only its speed does:
 the register kernel (one thread per cell, the whole state in registers;
-unordered sets of at most 256 cells) or the memory-state kernel with a CTA
+unordered sets, of at most 256 cells on one CTA and of up to 4096 over a
+cluster of CTAs) or the memory-state kernel with a CTA
 of 32..256 threads (any set; cells beyond the CTA width loop, so the CTA
 size is the cells-per-thread knob), or for sets with in-order neighbour
 reads the wave kernel, whose CTA holds one thread group per time step in
@@ -15,7 +16,8 @@ or not) and cell count (powers of two), times every candidate schedule of
 a bucket on a sample of its sets replicated to fill the GPU for a short
 horizon, and stamps the fastest schedule on every set of the bucket
 (ParameterSet.schedule / .mem_block).  Choices are cached per
-(model, bucket, GPU name) in a JSON file when one is given.
+(model, bucket, GPU name, version of the schedules) in a JSON file when one
+is given.
 """
 
 import copy
@@ -28,6 +30,9 @@ import numpy as np
 from . import engine as E
 
 MEM_BLOCKS = (32, 64, 128, 256)
+# part of a cached choice's key; raised when a kernel joins or changes, so
+# that choices made among others are made again
+SCHEDULES_VERSION = 2
 
 
 def bucket_of(s, levels):
@@ -37,7 +42,8 @@ def bucket_of(s, levels):
 
 
 def candidates(ordered, cells_log2):
-    """Schedules worth timing for a bucket: (schedule, mem_block) pairs.
+    """Schedules that keep a set on one CTA worth timing for a bucket:
+    (schedule, mem_block) pairs.
     Ordered sets: the wave kernel with the engine's CTA (one thread group
     per step in flight) or one or two warps (fewer steps in flight, more
     sets per SM), only the neighbour-read species in shared memory, or
@@ -50,6 +56,15 @@ def candidates(ordered, cells_log2):
     out = [(E.SCHEDULE_AUTO, 0)] if cells <= 256 else []
     out += [(E.SCHEDULE_MEMORY, b) for b in MEM_BLOCKS if b <= max(32, cells)]
     return out
+
+
+def schedules(ordered, cells_log2):
+    """Every schedule worth timing for a bucket: candidates(), and for
+    unordered sets of 257 to 4096 cells, the engine's own choice first: the
+    register kernel over a cluster of CTAs (96 sets of 733 cells, 200 steps:
+    2.7 ms, the memory kernel 4.8)."""
+    cluster = [(E.SCHEDULE_AUTO, 0)] if not ordered and 256 < 1 << cells_log2 <= 4096 else []
+    return cluster + candidates(ordered, cells_log2)
 
 
 def _with(s, schedule, mem_block, duration):
@@ -110,7 +125,7 @@ class Autotuner:
         if self.gpu_name is None:
             import torch
             self.gpu_name = torch.cuda.get_device_name(self.device)
-        return "%s|%s|%d|%d" % (self.gpu_name, model, bucket[0], bucket[1])
+        return "%s|%s|%d|%d|%d" % (self.gpu_name, model, bucket[0], bucket[1], SCHEDULES_VERSION)
 
     def tune(self, model, sets, step_size):
         """Stamp the fastest schedule of each bucket on `sets` (in place);
@@ -131,7 +146,7 @@ class Autotuner:
                 pick = rng.choice(idx, size=min(self.sample_sets, len(idx)), replace=False)
                 sample = [sets[i] for i in pick]
                 results = []
-                cands = candidates(bucket[0], bucket[1])
+                cands = schedules(bucket[0], bucket[1])
                 for cand in cands if len(cands) > 1 else []:
                     v = self.timer(model, sample, cand[0], cand[1], step_size, self.minutes, device=self.device)
                     results.append((v, cand))
