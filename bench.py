@@ -306,9 +306,13 @@ def run_mixed(a):
     achieved = done_bytes / (total_ms / 1e3) / 1e9
     cpu = mixed_cpu_sample(groups) if (rank == 0 and world == 1 and not a.no_cpu) else None
     if rank == 0:
-        from dense_b200.engine import plan
-        # one launch per kernel group of each engine (register kernel, one per memory-kernel CTA size)
-        n_launch = sum(len(set(plan(m, b.sets, 0.01, 1.0)[1].tolist())) for m, b in mb.batches.items())
+        from dense_b200.engine import plan, plan_ctas
+        # one launch per kernel group of each engine (register kernel, one per cluster size and its CTA size,
+        # one per memory-kernel CTA size)
+        n_launch = 0
+        for m, b in mb.batches.items():
+            kinds = zip(b.sets, plan(m, b.sets, 0.01, 1.0)[1].tolist(), plan_ctas(m, b.sets, 0.01, 1.0).tolist())
+            n_launch += len({(c, k if c == 1 else -(-s.num_cells // c // 32)) for s, k, c in kinds})
         line = {
             "metric": METRIC, "value": value, "unit": "cell-steps/s", "n_gpus": world, "steps": a.steps,
             "warmup": a.warmup, "ms_per_step": total_ms_max / a.steps, "higher_is_better": True, "scaling": "weak",

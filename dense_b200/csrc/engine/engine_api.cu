@@ -528,6 +528,20 @@ int plan_set(const dense_set_desc& in, double dt, int elem_bytes, SetPlan& plan,
   return DENSE_OK;
 }
 
+// Shared memory of a cluster CTA's sampled state: a row of every species that
+// some analysis observes.
+size_t cluster_sample_bytes(const std::vector<AnalysisDesc>& analyses) {
+  bool sampled[NUM_SPECIES] = {};
+  size_t bytes = 0;
+  for (const AnalysisDesc& A : analyses)
+    for (int i = 0; i < A.nsp; ++i)
+      if (!sampled[A.sp[i]]) {
+        sampled[A.sp[i]] = true;
+        bytes += sizeof(double) * (kStepThreads + kValsPad);
+      }
+  return bytes;
+}
+
 // Dynamic shared memory of a wave-kernel launch group holding a set that
 // needs `bytes`: a few fixed sizes, so sets of similar size share a launch.
 int wave_smem_bucket(int bytes) {
@@ -608,14 +622,7 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
   std::vector<uint16_t> rec_all;  // wave-kernel cell records, 8 x 16 bits each
   e->sets.resize(num_sets);
   e->init_status.resize(num_sets);
-  bool sampled[NUM_SPECIES] = {};
-  size_t sample_bytes = 0;  // shared memory of a cluster CTA's sampled state
-  for (const AnalysisDesc& A : e->analyses)
-    for (int i = 0; i < A.nsp; ++i)
-      if (!sampled[A.sp[i]]) {
-        sampled[A.sp[i]] = true;
-        sample_bytes += sizeof(double) * (kStepThreads + kValsPad);
-      }
+  const size_t sample_bytes = cluster_sample_bytes(e->analyses);
   std::vector<double> cp;
   for (int s = 0; s < num_sets; ++s) {
     const dense_set_desc& in = in_sets[s];
@@ -1194,8 +1201,8 @@ int dense_engine_ring_info(dense_engine* e, int set, int* S, int* D) {
 
 // Per-set device bytes and kernel of a batch, from the same planning as
 // dense_engine_create, without touching the GPU.
-int dense_engine_plan(const dense_run_desc* run, int num_sets, const dense_set_desc* in_sets, int64_t* set_bytes,
-                      int* set_kernel, int* set_levels) {
+static int plan_batch(const dense_run_desc* run, int num_sets, const dense_set_desc* in_sets, int64_t* set_bytes,
+                      int* set_kernel, int* set_levels, int* set_ctas) {
   if (!run || num_sets <= 0 || !in_sets) return fail(DENSE_ERR_INVALID, "null argument or no sets");
   if (!(run->step_size > 0.0) || !(run->analysis_interval > 0.0))
     return fail(DENSE_ERR_INVALID, "step size and analysis interval must be positive");
@@ -1225,8 +1232,19 @@ int dense_engine_plan(const dense_run_desc* run, int num_sets, const dense_set_d
                      (plan.wave ? 16 * n : 0);
     if (set_kernel) set_kernel[s] = plan.use_mem ? plan.mem_block : 0;
     if (set_levels) set_levels[s] = plan.d.ordered ? static_cast<int>(plan.lvl_off.size()) - 1 : 1;
+    if (set_ctas) set_ctas[s] = cluster_sample_bytes(analyses) <= kClusterSmem ? std::max(plan.ranks, 1) : 1;
   }
   return DENSE_OK;
+}
+
+int dense_engine_plan(const dense_run_desc* run, int num_sets, const dense_set_desc* sets, int64_t* set_bytes,
+                      int* set_kernel, int* set_levels) {
+  return plan_batch(run, num_sets, sets, set_bytes, set_kernel, set_levels, nullptr);
+}
+
+int dense_engine_plan_ctas(const dense_run_desc* run, int num_sets, const dense_set_desc* sets, int* set_ctas) {
+  if (!set_ctas) return fail(DENSE_ERR_INVALID, "null argument");
+  return plan_batch(run, num_sets, sets, nullptr, nullptr, nullptr, set_ctas);
 }
 
 // One CUDA graph over several engines (of any models' libraries): each

@@ -259,8 +259,8 @@ def _describe(L, sets, analyses, step_size, analysis_interval, precision, device
 
 
 def plan(model, sets, step_size, analysis_interval, analyses=(), precision=FP64):
-    """Per-set device bytes, kernel (0 = register kernel, else the
-    memory-state kernel's CTA size) and dependency levels per step (1 unless
+    """Per-set device bytes, kernel (0 = register kernel on one CTA, else the
+    memory-state or wave kernel's CTA size; see plan_ctas) and dependency levels per step (1 unless
     the set has ordered neighbour reads) that a Batch of these sets would
     use; needs no GPU."""
     L = load(model) if isinstance(model, str) else model
@@ -272,6 +272,21 @@ def plan(model, sets, step_size, analysis_interval, analyses=(), precision=FP64)
     L._check(L.lib.dense_engine_plan(C.byref(run), len(sets), cset, nbytes.ctypes.data_as(C.POINTER(C.c_int64)),
                                      _ip(kernel), _ip(levels)))
     return nbytes, kernel, levels
+
+
+def plan_ctas(model, sets, step_size, analysis_interval, analyses=(), precision=FP64):
+    """The CTAs each set is spread over: 1, or for unordered sets of 257 to
+    4096 cells the size of the cluster that runs them in the register kernel
+    (in the memory-state kernel of plan() on a GPU that holds no such
+    cluster); needs no GPU."""
+    L = load(model) if isinstance(model, str) else model
+    sets = list(sets)
+    run, cset, keep = _describe(L, sets, list(analyses), step_size, analysis_interval, precision, 0)
+    ctas = np.zeros(len(sets), np.int32)
+    f = L.lib.dense_engine_plan_ctas  # (not in libraries built before it)
+    f.restype, f.argtypes = C.c_int, [C.POINTER(_RunDesc), C.c_int, C.POINTER(_SetDesc), _I]
+    L._check(f(C.byref(run), len(sets), cset, _ip(ctas)))
+    return ctas
 
 
 class Batch:

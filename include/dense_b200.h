@@ -63,7 +63,8 @@ extern "C" {
 #define DENSE_SET_ORDERED_READS 16 /* neighbour reads of rows written in the same step */
 
 /* schedule hint of a set (dense_set_desc.schedule) */
-#define DENSE_SCHEDULE_AUTO 0              /* register kernel when the set fits one, else memory kernel */
+#define DENSE_SCHEDULE_AUTO 0              /* register kernel (up to 256 cells on one CTA, up to 4096 over a
+                                              cluster) when the set fits it, else memory kernel */
 #define DENSE_SCHEDULE_MEMORY 1            /* memory-state kernel; sets with in-order neighbour reads in
                                               the wave kernel, rows in shared memory as far as they fit */
 #define DENSE_SCHEDULE_GLOBAL 2            /* memory-state kernel with every row in global memory */
@@ -282,13 +283,20 @@ DENSE_API int dense_graph_destroy(void* graph_exec);
 /* Planning without a GPU (no counterpart in DENSE, whose Simulation objects
    size themselves, sim/base.cpp:55-140): per set, the device bytes
    dense_engine_create would hold for it (set_bytes, or NULL) and the kernel
-   it would run in (set_kernel: 0 = register kernel, else the memory-state
-   kernel's threads per CTA; or NULL) and the dependency levels of one of
+   it would run in (set_kernel: 0 = register kernel on one CTA, else the
+   memory-state or wave kernel's threads per CTA; or NULL) and the dependency levels of one of
    its steps (set_levels: 1 unless neighbour reads see rows written in the
    same step, DENSE's in-order cell loop; or NULL).  Used to size waves and
    to bucket sets for schedule tuning. */
 DENSE_API int dense_engine_plan(const dense_run_desc* run, int num_sets, const dense_set_desc* sets,
                                 int64_t* set_bytes, int* set_kernel, int* set_levels);
+
+/* The CTAs a set is spread over (1: one CTA): unordered sets of 257 to 4096
+   cells without a schedule hint run in the register kernel over a cluster of
+   so many CTAs on a GPU that holds such a cluster, and only on another in
+   the memory-state kernel with the threads that dense_engine_plan gives. */
+DENSE_API int dense_engine_plan_ctas(const dense_run_desc* run, int num_sets, const dense_set_desc* sets,
+                                     int* set_ctas);
 
 /* No counterpart in DENSE: an addition of this library for callers that may
    not allocate device memory -- code running inside a framework that owns
