@@ -328,6 +328,9 @@ struct RegContext {
     if (kMode == kChecked) return own_checked(sp, d.k);
     const int i = d.dr * kNS + sp;
     if (kMode == kUse && f->has_own[i]) return f->own[i];
+    // (a read that the fetch pass did not come to, behind a condition that
+    // turned out otherwise there, is late: nothing looks at `seen` any more)
+    if (kMode == kUse && (own_at[i] & kReadCheckBit)) return own_checked(sp, d.k);
     const T v = fetch_own(sp, own_at[i]);
     f->own[i] = v;
     f->has_own[i] = true;
@@ -338,6 +341,7 @@ struct RegContext {
     if (kMode == kChecked) return nbr_checked(sp, d.k);
     const int i = d.dr * kNS + sp;
     if (kMode == kUse && f->has_nbr[i]) return f->nbr[i];
+    if (kMode == kUse && (nbr_at[i] & kReadCheckBit)) return nbr_checked(sp, d.k);
     const T v = fetch_nbr(sp, nbr_at[i]);
     f->nbr[i] = v;
     f->has_nbr[i] = true;
