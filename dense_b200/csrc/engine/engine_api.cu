@@ -710,7 +710,7 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
     e->sets[s] = d;
   }
 
-  // ---- device buffers: what the host writes first, in one upload
+  // ---- device buffers: what the host writes first
   const size_t tsz = run->precision == DENSE_FP64 ? sizeof(double) : sizeof(float);
   int rc;
   if (mem_list.empty()) std::vector<int>().swap(lvl_cells_all);  // only the memory kernel reads cells in level order
@@ -733,11 +733,11 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
                   {&e->d_ring, tsz * ring_total, 0},
                   {&e->d_anl, sizeof(double) * anl_block * num_sets, 0}};
   constexpr int kUploads = 10;  // the first parts
-  size_t total = 0, upload = 0;
+  constexpr size_t kStagedPart = size_t(1) << 20;  // bytes of a part that is staged with its neighbours
+  size_t total = 0;
   for (int i = 0; i < static_cast<int>(sizeof parts / sizeof parts[0]); ++i) {
     parts[i].at = total;
     total += (std::max<size_t>(parts[i].bytes, 16) + 255) & ~size_t(255);
-    if (i + 1 == kUploads) upload = total;
   }
   if ((rc = e->d_all.alloc(total))) return rc;
   for (Part& x : parts) x.b->view(static_cast<char*>(e->d_all.p) + x.at, x.bytes);
@@ -811,7 +811,9 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
     }
   }
   {
-    // staged in one block and copied at once
+    // neighbouring small parts staged in one block and copied at once, large
+    // ones (per-cell parameters: 0.3 GB for 4096 sets of 200 cells) from
+    // where they are
     std::vector<int> lists(reg_list);
     lists.insert(lists.end(), mem_list.begin(), mem_list.end());
     std::vector<float> params_f;
@@ -821,10 +823,23 @@ int dense_engine_create(const dense_run_desc* run, int num_sets, const dense_set
                                                                      : params_f.data(),
                                         off_all.data(), idx_all.data(), conc_all.data(), e->init_status.data(),
                                         lists.data(), lvl_off_all.data(), lvl_cells_all.data(), rec_all.data()};
-    std::vector<unsigned char> staged(upload);
-    for (int i = 0; i < kUploads; ++i)
-      if (parts[i].bytes > 0) std::memcpy(staged.data() + parts[i].at, from[i], parts[i].bytes);
-    CUDA_TRY(cudaMemcpyAsync(e->d_all.p, staged.data(), upload, cudaMemcpyHostToDevice, e->stream));
+    unsigned char* const base = static_cast<unsigned char*>(e->d_all.p);
+    std::vector<std::vector<unsigned char>> staged;
+    for (int i = 0; i < kUploads;) {
+      if (parts[i].bytes > kStagedPart) {
+        CUDA_TRY(cudaMemcpyAsync(base + parts[i].at, from[i], parts[i].bytes, cudaMemcpyHostToDevice, e->stream));
+        ++i;
+        continue;
+      }
+      const int first = i;
+      while (i < kUploads && parts[i].bytes <= kStagedPart) ++i;
+      const size_t begin = parts[first].at, end = parts[i - 1].at + parts[i - 1].bytes;
+      if (end == begin) continue;
+      staged.emplace_back(end - begin);
+      for (int k = first; k < i; ++k)
+        if (parts[k].bytes > 0) std::memcpy(staged.back().data() + (parts[k].at - begin), from[k], parts[k].bytes);
+      CUDA_TRY(cudaMemcpyAsync(base + begin, staged.back().data(), end - begin, cudaMemcpyHostToDevice, e->stream));
+    }
     CUDA_TRY(cudaStreamSynchronize(e->stream));
   }
   e->device_bytes = static_cast<int64_t>(e->d_sets.bytes + e->d_prog.bytes + e->d_params.bytes + e->d_nbr_off.bytes +
