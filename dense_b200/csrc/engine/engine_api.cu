@@ -108,7 +108,8 @@ void plan_levels(const dense_set_desc& in, bool ordered, SetPlan& plan) {
 // and drops a batch per generation.  Allocations of up to kPoolKeep come
 // from a stream-ordered pool of the device that keeps at most kPoolKeep
 // (0.3 % of the GPU's memory) mapped once they are freed (1 us each then);
-// larger ones, and any the pool cannot serve, are plain cudaMalloc.  The
+// larger ones, and any the pool cannot serve, are plain cudaMalloc, for which
+// the pool gives back what it keeps when the device has no room.  The
 // pool is the driver's own object: calls from several threads are safe, and
 // an allocation is freed only after the device has been synchronised, so no
 // stream can still use it.
@@ -170,21 +171,26 @@ struct DeviceBuffer {
     bytes = n;
     if (n == 0) n = 16;
     int device = 0;
-    if (n <= kPoolKeep && cudaGetDevice(&device) == cudaSuccess) {
-      const DevicePool pool = device_pool(device);
-      if (pool.pool) {
-        // (synchronised, so usable on every stream)
-        if (cudaMallocFromPoolAsync(&p, n, pool.pool, pool.stream) == cudaSuccess &&
-            cudaStreamSynchronize(pool.stream) == cudaSuccess) {
-          pool_stream = pool.stream;
-          return DENSE_OK;
-        }
-        p = nullptr;
-        cudaGetLastError();
-        cudaMemPoolTrimTo(pool.pool, 0);
+    DevicePool pool;
+    if (cudaGetDevice(&device) == cudaSuccess) pool = device_pool(device);
+    if (n <= kPoolKeep && pool.pool) {
+      // (synchronised, so usable on every stream)
+      if (cudaMallocFromPoolAsync(&p, n, pool.pool, pool.stream) == cudaSuccess &&
+          cudaStreamSynchronize(pool.stream) == cudaSuccess) {
+        pool_stream = pool.stream;
+        return DENSE_OK;
       }
+      p = nullptr;
+      cudaGetLastError();
     }
     cudaError_t e = cudaMalloc(&p, n);
+    if (e == cudaErrorMemoryAllocation && pool.pool) {
+      // what the pool keeps of batches dropped before may be what is missing
+      cudaGetLastError();
+      cudaStreamSynchronize(pool.stream);
+      cudaMemPoolTrimTo(pool.pool, 0);
+      e = cudaMalloc(&p, n);
+    }
     if (e != cudaSuccess) {
       p = nullptr;
       return fail(DENSE_ERR_MEMORY, std::string("cudaMalloc(") + std::to_string(n) + "): " + cudaGetErrorString(e));
