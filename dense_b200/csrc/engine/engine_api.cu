@@ -24,7 +24,6 @@
 #include <cstring>
 #include <map>
 #include <memory>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -33,6 +32,7 @@
 #include "model_impl.hpp"
 
 #include "dense_b200.h"
+#include "device_pool.hpp"
 #include "engine_launch.hpp"
 #include "engine_types.hpp"
 #include "lag_trace.hpp"
@@ -100,49 +100,6 @@ void plan_levels(const dense_set_desc& in, bool ordered, SetPlan& plan) {
   std::vector<int> fill(plan.lvl_off.begin(), plan.lvl_off.end() - 1);
   for (int c = 0; c < n; ++c) plan.lvl_cells[fill[level[c]]++] = c;
   plan.d.n_levels = n_levels;
-}
-
-// Device memory kept for the next batch.  cudaMalloc and cudaFree of more
-// than the driver's 2 MB chunks map and unmap memory: 0.3-1 ms and 0.3-3 ms
-// here (1 MB to 256 MB), as much as a small batch's run, and a search makes
-// and drops a batch per generation.  Allocations of up to kPoolKeep come
-// from a stream-ordered pool of the device that keeps at most kPoolKeep
-// (0.3 % of the GPU's memory) mapped once they are freed (1 us each then);
-// larger ones, and any the pool cannot serve, are plain cudaMalloc, for which
-// the pool gives back what it keeps when the device has no room.  The
-// pool is the driver's own object: calls from several threads are safe, and
-// an allocation is freed only after the device has been synchronised, so no
-// stream can still use it.
-constexpr size_t kPoolKeep = size_t(512) << 20;
-
-struct DevicePool {
-  cudaMemPool_t pool = nullptr;
-  cudaStream_t stream = nullptr;  // orders the pool's allocations and frees
-};
-
-DevicePool device_pool(int device) {
-  constexpr int kMaxDevices = 64;
-  static std::mutex mu;
-  static DevicePool pools[kMaxDevices];
-  static bool tried[kMaxDevices] = {};
-  if (device < 0 || device >= kMaxDevices) return {};
-  std::lock_guard<std::mutex> lock(mu);
-  if (!tried[device]) {
-    tried[device] = true;
-    cudaMemPoolProps props{};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = device;
-    DevicePool made;
-    uint64_t keep = kPoolKeep;
-    if (cudaMemPoolCreate(&made.pool, &props) == cudaSuccess &&
-        cudaMemPoolSetAttribute(made.pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess &&
-        cudaStreamCreateWithFlags(&made.stream, cudaStreamNonBlocking) == cudaSuccess)
-      pools[device] = made;
-    else
-      cudaGetLastError();
-  }
-  return pools[device];
 }
 
 struct DeviceBuffer {

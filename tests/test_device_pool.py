@@ -50,3 +50,18 @@ def test_the_pool_keeps_at_most_half_a_gigabyte(count, tmp_path):
     log = calls(MAKE + "a = batch(%d)\nb = batch(%d)\na.close()\nb.close()\n" % (count, count), tmp_path)
     held = [int(x.split()[3]) for x in log if x.startswith("pool_free")]
     assert len(held) == 2 and held[-1] <= 512 * MB
+
+
+def test_models_share_one_pool_per_device(tmp_path):
+    """Each model is a library of its own; the memory that they keep together
+    is bounded."""
+    log = calls(MAKE + """
+from tests.test_wave_gpu import _grid
+grid = N.engine_library(N.GRID)
+for device in (0, 1):
+    E.Batch(lib, _sets(200, False, 1, count=1) * 20, 0.01, 0.1, [], device=device).close()
+    E.Batch(grid, _grid(100, 10, 3, duration=2.0), 0.01, 0.1, [], device=device).close()
+""", tmp_path)
+    assert [x for x in log if x.startswith("pool dev")] == ["pool dev 0", "pool dev 1"]
+    sizes, held = _sizes(log, "pool_malloc"), [int(x.split()[3]) for x in log if x.startswith("pool_free")]
+    assert sizes[1] < sizes[0] and held[0] == held[1]  # the second model's batch is served from what the first left
