@@ -326,6 +326,26 @@ class MLP:
         self.k.pack(self.W, self._packed, backward)
         return self._packed
 
+    def forward(self, Xb):
+        """Outputs [Bp][OUT_PAD] (float32) of padded BF16 rows Xb [Bp][IN_PAD],
+        Bp a multiple of 128, a GEMM a layer: for callers that want the
+        layers' own outputs, self.Z (before GELU) and self.H (after; H[0] is
+        Xb) besides.  The buffers are this object's and are written again by
+        the next call of the same size."""
+        bf = self.torch.bfloat16
+        Bp = Xb.shape[0]
+        self.Z = [self._buf("Z%d" % i, (Bp, HIDDEN)) for i in range(3)]
+        self.H = [Xb] + [self._buf("H%d" % i, (Bp, HIDDEN), bf) for i in range(1, 4)]
+        Y = self._buf("Y", (Bp, OUT_PAD))
+        for i, w in enumerate(self.W):
+            Wb = self._buf("Wb%d" % i, w.shape, bf)
+            self.k.cast(w, Wb)
+            if i < 3:
+                self.k.gemm(self.H[i], Wb, self.Z[i], EPI_BIAS_GELU, self.b[i], self.H[i + 1])
+            else:
+                self.k.gemm(self.H[3], Wb, Y, EPI_BIAS, self.b[3])
+        return Y
+
     def _rows(self, X):
         """Float32 CUDA rows [B][n_in] of X, each value rounded as it would
         be to BF16 (once)."""
