@@ -221,8 +221,9 @@ class Kernels:
         """out [rows][n_out] of the packed network for float32 rows X."""
         n, n_in = X.shape
         assert X.stride(1) == 1 or n_in == 1
-        assert self.L.dense_mlp_predict(_p(X), max(X.stride(0), n_in), n, n_in, _p(packed), _pp(bias), out.shape[1],
-                                        _p(out), _p(self.err), self._s()) == 0
+        ld = X.stride(0) if n > 1 else n_in  # (the stride of a single row is no leading dimension)
+        assert self.L.dense_mlp_predict(_p(X), ld, n, n_in, _p(packed), _pp(bias), out.shape[1], _p(out),
+                                        _p(self.err), self._s()) == 0
 
     def rank(self, P, idx, tmpl, log_spread, packed, biases, n_out, mu, sd, weight, period, tol, amp_min, ramp, out):
         """Ranking scores of candidates P (float64 [n][params]) under the
@@ -346,6 +347,13 @@ class MLP:
                 self.k.gemm(self.H[3], Wb, Y, EPI_BIAS, self.b[3])
         return Y
 
+    def _as_rows(self, X):
+        """Whether X is float32 rows [B][n_in] that the kernels read as they
+        are (the leading dimension is a C int)."""
+        return (X.dtype == self.torch.float32 and X.device == self.dev and X.shape[1] == self.n_in and
+                (X.stride(1) == 1 or self.n_in == 1) and
+                (X.shape[0] <= 1 or self.n_in <= X.stride(0) < 2 ** 31))
+
     def _rows(self, X):
         """Float32 CUDA rows [B][n_in] of X, each value rounded as it would
         be to BF16 (once)."""
@@ -354,15 +362,18 @@ class MLP:
         if X.dtype != torch.float32:
             X = X.to(torch.bfloat16).to(torch.float32)
         X = X.to(self.dev).expand(X.shape[0], self.n_in)
-        return X if X.stride(1) == 1 and X.stride(0) >= self.n_in else X.contiguous()
+        return X if self._as_rows(X) else X.contiguous()
 
     def predict_device(self, X, batch=65536):
         """Outputs [B][n_out] as a CUDA float32 tensor, for inputs already
         on the GPU (a float tensor [B][n_in]); nothing crosses to the host.
-        One launch carries every row through the whole network (`batch` is
-        kept for callers that pass it)."""
+        One launch carries every row through the whole network; inputs of
+        another type or layout are converted `batch` rows at a time."""
         out = self.torch.empty((X.shape[0], self.n_out), device=self.dev)
-        self.k.predict(self._rows(X), self._pack(), self.b, out)
+        packed = self._pack()
+        step = max(1, X.shape[0]) if self._as_rows(X) else batch
+        for s in range(0, X.shape[0], step):
+            self.k.predict(self._rows(X[s:s + step]), packed, self.b, out[s:s + step])
         self.k.check()
         return out
 
