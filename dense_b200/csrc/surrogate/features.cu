@@ -64,6 +64,12 @@ struct CellStats {
   double n, mean, m2;
   __device__ __forceinline__ void join(double bn, double bmean, double bm2) {
     if (bn <= 0.0) return;
+    if (n <= 0.0) {  // (the update's square of bmean may be out of range)
+      n = bn;
+      mean = bmean;
+      m2 = bm2;
+      return;
+    }
     const double total = n + bn, w = bn / total, d = bmean - mean;
     mean += d * w;
     m2 += bm2 + d * d * (n * w);
@@ -132,7 +138,7 @@ __global__ void __launch_bounds__(kSyncThreads, 2) synchrony_kernel(const double
       // CellStats::join of equal blocks: k blocks and one more
       const double w = k < kSyncInv ? s_inv[k] : 1.0 / (k + 1), d = m - mean;
       mean += d * w;
-      m2 += (q0 + q1) + d * d * (8.0 * k * w);
+      m2 += (q0 + q1) + (k > 0 ? d * d * (8.0 * k * w) : 0.0);
     }
     CellStats st{8.0 * k, mean, m2};
     for (int j = 0; t + j < rows && j < 8; ++j) {
@@ -167,8 +173,10 @@ __global__ void __launch_bounds__(kSyncThreads, 2) synchrony_kernel(const double
     const double nrm = sqrt(st.m2);
     const bool ok = nrm > 1e-12 * (1.0 + largest);
     centre[c] = st.mean;
-    s_mean[c] = ok ? nrm : 0.0;  // the groups' statistics are done with: now the norms (0: left out)
-    s_m2[c] = ok ? 1.0 / nrm : 0.0;  // and their reciprocals
+    // the groups' statistics are done with: now the norms (0: left out) and
+    // their reciprocals (a norm out of range: quotients of 0)
+    s_mean[c] = ok ? (isinf(nrm) ? 1.0 : nrm) : 0.0;
+    s_m2[c] = ok ? 1.0 / nrm : 0.0;
     n_ok += ok ? 1.0 : 0.0;
   }
   const double n = block_sum(n_ok, red);  // (its barriers also publish the norms)
