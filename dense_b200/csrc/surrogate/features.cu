@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(kSyncThreads, 2) synchrony_kernel(const double
   double* centre = r_m2 + cells;                            // the cells' means over every rank
   __shared__ int share_top;
   __shared__ double share_sq;
+  __shared__ unsigned long long share_bits;
   __shared__ double s_inv[kSyncInv];                        // 1 / (k + 1)
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
@@ -109,8 +110,8 @@ __global__ void __launch_bounds__(kSyncThreads, 2) synchrony_kernel(const double
   int width = 32;
   while (width < cells && width < threads) width *= 2;
   const int groups = threads / width, grp = tid / width, first = tid % width;
-  // largest magnitude, to the 20 mantissa bits of its upper word (it only
-  // scales the test for constant traces); infinities and NaN lie above all
+  // largest magnitude, to the 20 mantissa bits of its upper word (exactly
+  // below, where the rest decides); infinities and NaN lie above all
   int top = 0;
   auto magnitude = [&](double v) { top = max(top, __double2hiint(v) & 0x7fffffff); };
   for (int i = tid; i < kSyncInv; i += threads) s_inv[i] = 1.0 / (i + 1);
@@ -161,9 +162,15 @@ __global__ void __launch_bounds__(kSyncThreads, 2) synchrony_kernel(const double
   if (lane == 0) atomicMax(&share_top, top);
   cluster.sync();
   for (int k = 0; k < ranks; ++k) top = max(top, *cluster.map_shared_rank(&share_top, k));
-  // with an infinite or NaN sample no cell counts (the comparison fails)
-  const double largest = __hiloint2double(top, 0);
-  double n_ok = 0.0;
+  // The largest magnitude scales the threshold of a constant trace.  Between
+  // the least and the greatest value of its upper word no norm lies but by
+  // rare chance: then it is looked up exactly (every CTA of the cluster has
+  // the same norms and comes to the same decision).  With an infinite or NaN
+  // sample no cell counts (the comparison fails).
+  double largest = __hiloint2double(top, 0);
+  const double most = __hiloint2double(top, -1);
+  auto counts_with = [](double nrm, double magnitude_) { return nrm > 1e-12 * (1.0 + magnitude_); };
+  bool unsure = false;
   for (int c = tid; c < cells; c += threads) {
     CellStats st{0.0, 0.0, 0.0};
     for (int k = 0; k < ranks; ++k) {
@@ -171,10 +178,27 @@ __global__ void __launch_bounds__(kSyncThreads, 2) synchrony_kernel(const double
       st.join(rk, cluster.map_shared_rank(r_mean, k)[c], cluster.map_shared_rank(r_m2, k)[c]);
     }
     const double nrm = sqrt(st.m2);
-    const bool ok = nrm > 1e-12 * (1.0 + largest);
     centre[c] = st.mean;
-    // the groups' statistics are done with: now the norms (0: left out) and
-    // their reciprocals (a norm out of range: quotients of 0)
+    s_mean[c] = nrm;  // the groups' statistics are done with
+    unsure = unsure || (counts_with(nrm, largest) && !counts_with(nrm, most));
+  }
+  if (__syncthreads_or(unsure) && top < 0x7ff00000) {
+    unsigned long long bits = 0;
+    const double* all = X + set * set_stride;
+    for (int64_t i = tid; i < static_cast<int64_t>(T) * cells; i += threads)
+      bits = max(bits, __double_as_longlong(all[i / cells * sample_stride + i % cells]) & 0x7fffffffffffffffull);
+    if (tid == 0) share_bits = 0;
+    __syncthreads();
+    atomicMax(&share_bits, bits);
+    __syncthreads();
+    largest = __longlong_as_double(share_bits);
+  }
+  // the norms (0: left out) and their reciprocals (a norm out of range:
+  // quotients of 0)
+  double n_ok = 0.0;
+  for (int c = tid; c < cells; c += threads) {
+    const double nrm = s_mean[c];
+    const bool ok = counts_with(nrm, largest);
     s_mean[c] = ok ? (isinf(nrm) ? 1.0 : nrm) : 0.0;
     s_m2[c] = ok ? 1.0 / nrm : 0.0;
     n_ok += ok ? 1.0 : 0.0;

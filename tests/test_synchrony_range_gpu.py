@@ -32,3 +32,21 @@ def test_squares_out_of_range(mean, spread, samples):
     eps m, so a unit trace is known to eps m / spread."""
     X = np.stack([mean + spread * _traces(samples, 24, i) for i in range(3)])
     _check(X, 1e-12 + 8 * 2.2e-16 * abs(mean) / spread)
+
+
+@pytest.mark.parametrize("cells", [3, 40, 700])
+@pytest.mark.parametrize("samples", [16, 600])
+@pytest.mark.parametrize("above", [False, True])
+def test_cells_next_to_the_threshold(above, samples, cells):
+    """A cell counts when its norm is above 1e-12 (1 + the largest magnitude),
+    the whole of it: a magnitude's lower word moves the threshold by up to a
+    millionth."""
+    X = np.stack([_traces(samples, cells, i) for i in range(2)])
+    X[1, samples // 2, 2] = np.nextafter(4.0e6, 0.0)  # its lower word is all ones
+    top = np.abs(X[1]).max()
+    short = np.array(np.array(top).view(np.uint64) & np.uint64(0xFFFFFFFF00000000)).view(np.float64)[()]
+    assert top > short
+    norm = 1e-12 * (1.0 + (top * (1 + 1e-8) if above else 0.5 * (top + short)))
+    half = norm / np.sqrt(samples)
+    X[1, :, 0] = np.where(np.arange(samples) % 2, half, -half)
+    _check(X)
