@@ -197,7 +197,9 @@ __device__ __forceinline__ int layer_of(int i, int* within) {
   if (i < s2) return *within = i - s1, 2;
   return *within = i - s2, 3;
 }
-constexpr int kWeights = kHid * kInPad + 2 * kHid * kHid + kOutPad * kHid;
+constexpr int kOutWeights = kOutPad * kHid;
+constexpr int kHidWeights = kHid * kInPad + 2 * kHid * kHid;
+constexpr int kWeights = kHidWeights + kOutWeights;
 
 // Four consecutive weights of a row at a time.
 __device__ __forceinline__ void pack_quad(unsigned char* packed, int layer, int at, const float (&w)[4], bool backward) {
@@ -1022,8 +1024,10 @@ struct WgradArgs {
   const unsigned char *act, *grad;
   int64_t blocks;   // 64-row blocks of the batch
   int oc;           // 64-column chunks of dY
-  int splits, per;  // ranges of `per` blocks
-  float* parts;     // [splits][kWeights]
+  int splits, per;          // layers 0-2: ranges of `per` blocks
+  int out_splits, out_per;  // the output layer's
+  float* parts;             // [splits][kHidWeights]
+  float* out_parts;         // [out_splits][kOutWeights]
   int* err;
 };
 
@@ -1042,14 +1046,16 @@ __global__ void __launch_bounds__(kWgradThreads, 1) mlp_wgrad_kernel(const Wgrad
   __shared__ volatile int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   unsigned char* ring = wgrad_raw + ((1024u - (smem_u32(wgrad_raw) & 1023u)) & 1023u);
-  const int unit = blockIdx.x % 7, split = blockIdx.x / 7;
+  const bool output = static_cast<int>(blockIdx.x) >= 6 * a.splits;
+  const int unit = output ? 6 : blockIdx.x % 6, split = output ? blockIdx.x - 6 * a.splits : blockIdx.x / 6;
   const int layer = unit >> 1, half = unit & 1;
+  const int per = output ? a.out_per : a.per;
   const int n = layer == 0 ? kInPad : kHid;
   const int nc = n / 64;                            // chunks of the layer input
   const int ac = layer == 3 ? a.oc : 4;             // chunks of dZ
   const int take = layer == 3 ? a.oc : 2;           // of them, this unit's
-  const int64_t b0 = static_cast<int64_t>(split) * a.per;
-  const int count = static_cast<int>(a.blocks - b0 < a.per ? a.blocks - b0 : a.per);
+  const int64_t b0 = static_cast<int64_t>(split) * per;
+  const int count = static_cast<int>(a.blocks - b0 < per ? a.blocks - b0 : per);
 
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)), "r"(256));
@@ -1126,8 +1132,10 @@ __global__ void __launch_bounds__(kWgradThreads, 1) mlp_wgrad_kernel(const Wgrad
     if (mbar_wait_or(&acc_full, 0u, &abort_flag) && !abort_flag) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int o = half * 128 + q * 32 + lane;  // output row of the layer
-      constexpr int first[4] = {0, kHid * kInPad, kHid * kInPad + kHid * kHid, kHid * kInPad + 2 * kHid * kHid};
-      float* dst = a.parts + static_cast<int64_t>(split) * kWeights + first[layer] + static_cast<int64_t>(o) * n;
+      constexpr int first[3] = {0, kHid * kInPad, kHid * kInPad + kHid * kHid};
+      float* dst = (output ? a.out_parts + static_cast<int64_t>(split) * kOutWeights
+                           : a.parts + static_cast<int64_t>(split) * kHidWeights + first[layer]) +
+                   static_cast<int64_t>(o) * n;
       // rows of the output layer past dY's chunks have no gradient
       const bool live = layer < 3 || q * 32 + lane < a.oc * 64;
       for (int c = 0; c < n; c += 16) {
@@ -1210,9 +1218,10 @@ __global__ void __launch_bounds__(256) mlp_bias_sums_kernel(const float* dz, con
 // ------------------------------------------------------------------- finish
 
 struct FinishArgs {
-  const float* parts;    // [splits][kWeights]
-  const float* db_part;  // [4][8][256]
-  int splits, oc;
+  const float* parts;      // [splits][kHidWeights]
+  const float* out_parts;  // [out_splits][kOutWeights]
+  const float* db_part;    // [4][8][256]
+  int splits, out_splits, oc;
   float *dW[4], *db[4];  // written when dW[0] is not null
   // Adam, when hyper is not null: {lr, b1, b2, eps, 1 - b1^t, 1 - b2^t}
   const float* hyper;
@@ -1240,10 +1249,12 @@ __global__ void __launch_bounds__(256) mlp_finish_kernel(const __grid_constant__
   if (t < kWeights / 4) {
     int at;
     const int layer = layer_of(t * 4, &at);
-    const float4* p = reinterpret_cast<const float4*>(a.parts) + t;
+    const float4* p = reinterpret_cast<const float4*>(layer == 3 ? a.out_parts + at : a.parts + t * 4);
+    const int splits = layer == 3 ? a.out_splits : a.splits;
+    const int64_t stride = (layer == 3 ? kOutWeights : kHidWeights) / 4;
     float4 s = *p;
-    for (int k = 1; k < a.splits; ++k) {
-      const float4 x = p[static_cast<int64_t>(k) * (kWeights / 4)];
+    for (int k = 1; k < splits; ++k) {
+      const float4 x = p[k * stride];
       s.x += x.x;
       s.y += x.y;
       s.z += x.z;
@@ -1458,25 +1469,30 @@ CHAIN_API int dense_mlp_rank(const double* P, int ldp, int rows, const int* cols
 // activations, gradients, GELU' and the column sums, then the parts.
 namespace {
 struct TrainBuffers {
-  int64_t tiles, blocks, per, splits;
-  int64_t grad, dz, dy, db_part, parts, bytes;
+  int64_t tiles, blocks, per, splits, out_per, out_splits;
+  int64_t grad, dz, dy, db_part, parts, out_parts, bytes;
   TrainBuffers(int rows, int n_out) {
     tiles = (static_cast<int64_t>(rows) + kRows - 1) / kRows;
     blocks = 2 * tiles;
-    // ranges of four blocks or a little more (the bulk copies of a range are
-    // then all in flight; dense_mlp_gemm_ws splits the same products the
-    // same way), longer ones when seven units of each range would not fit
-    // the GPU's SMs at once
-    splits = blocks < 8 ? 1 : blocks / 4;
-    if (7 * splits > 148) splits = 148 / 7;
-    per = (blocks + splits - 1) / splits;
-    splits = (blocks + per - 1) / per;
+    // Ranges of four blocks or a little more (the bulk copies of a range are
+    // then all in flight), longer ones past as many ranges as one layer's
+    // units fill the GPU's SMs with: each FP32 sum runs over so many rows,
+    // the same as in dense_mlp_gemm_ws, whose results these equal.
+    auto ranges = [&](int64_t most, int64_t* n, int64_t* each) {
+      *n = blocks < 8 ? 1 : blocks / 4;
+      if (*n > most) *n = most;
+      *each = (blocks + *n - 1) / *n;
+      *n = (blocks + *each - 1) / *each;
+    };
+    ranges(148 / 2, &splits, &per);
+    ranges(148, &out_splits, &out_per);
     grad = 13 * blocks * kHalf;
     dz = grad + (12 + out_chunks(n_out)) * blocks * kHalf;
     dy = dz + 3 * tiles * kRows * kHid * 4;
     db_part = dy + tiles * kRows * out_chunks(n_out) * 64 * 4;
     parts = db_part + 4 * kColSlices * kHid * 4;
-    bytes = parts + splits * kWeights * 4;
+    out_parts = parts + splits * kHidWeights * 4;
+    bytes = out_parts + out_splits * kOutWeights * 4;
   }
 };
 }  // namespace
@@ -1543,9 +1559,12 @@ CHAIN_API int dense_mlp_train_pass(const float* X, int ldx, int x_rows, int n_in
   g.oc = out_chunks(n_out);
   g.splits = static_cast<int>(t.splits);
   g.per = static_cast<int>(t.per);
+  g.out_splits = static_cast<int>(t.out_splits);
+  g.out_per = static_cast<int>(t.out_per);
   g.parts = reinterpret_cast<float*>(w + t.parts);
+  g.out_parts = reinterpret_cast<float*>(w + t.out_parts);
   g.err = err;
-  return launch_next(mlp_wgrad_kernel, dim3(7 * g.splits), kWgradThreads, kWgradSmem, s, g) ? 2 : 0;
+  return launch_next(mlp_wgrad_kernel, dim3(6 * g.splits + g.out_splits), kWgradThreads, kWgradSmem, s, g) ? 2 : 0;
 }
 
 CHAIN_API int dense_mlp_train_finish(const void* work, int64_t work_bytes, int rows, int n_out, float* const* dW,
@@ -1560,8 +1579,10 @@ CHAIN_API int dense_mlp_train_finish(const void* work, int64_t work_bytes, int r
   const unsigned char* w = static_cast<const unsigned char*>(work);
   FinishArgs a{};
   a.parts = reinterpret_cast<const float*>(w + t.parts);
+  a.out_parts = reinterpret_cast<const float*>(w + t.out_parts);
   a.db_part = reinterpret_cast<const float*>(w + t.db_part);
   a.splits = static_cast<int>(t.splits);
+  a.out_splits = static_cast<int>(t.out_splits);
   a.oc = out_chunks(n_out);
   a.hyper = hyper;
   for (int i = 0; i < 4; ++i) {
