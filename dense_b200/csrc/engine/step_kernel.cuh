@@ -565,8 +565,9 @@ struct OscQueue : OscIndex {
 
 // OscillationAnalysis::checkCritPoint (oscillation.ipp:110-119): the middle
 // value is a peak when it equals the window's maximum and not its minimum,
-// a trough when it equals the minimum -- that is, a peak when no live value
-// lies above it and some lies below, a trough when none lies below.  The
+// a trough when it equals the minimum -- that is, where it is one of the live
+// values, a peak when none of them lies above it and some lies below, a
+// trough when none lies below.  The
 // window is scanned from both ends inwards, four values from each end at a
 // time, and the scan stops as soon as values above and below have both been
 // seen, so only an extreme middle value costs a whole pass -- and a flat
@@ -611,6 +612,21 @@ __device__ __forceinline__ void osc_check(const OscRef& o, const OscQueue& q, co
     left -= 8;
   }
   if (above && below) return;
+  // The middle slot may have been dequeued by now (windows of one, three or
+  // five samples, and ones that a run or a finalization left with a few):
+  // its value is then no longer among the live ones, and DENSE's extremum,
+  // one of them, need not equal it.
+  int ahead = q.current - q.start;
+  if (ahead < 0) ahead += w;
+  if (ahead >= q.live) {
+    bool equal = false;
+    int at = q.start;
+    for (int u = 0; u < q.live; ++u) {
+      equal = equal || win[static_cast<size_t>(at) * m] == mid;
+      at = (at == w - 1) ? 0 : at + 1;
+    }
+    if (!equal) return;
+  }
   double t = (samples - static_cast<double>(A.range_steps / 2)) * A.interval + A.t0;
   t = (0.0 < t) ? t : 0.0;
   if (!above && below) osc_add_crit(o, t, mid, true);
