@@ -582,6 +582,11 @@ __device__ __forceinline__ void osc_check(const OscRef& o, const OscQueue& q, co
   if (q.current < 0 || q.live <= 0) return;
   const double mid = win[static_cast<size_t>(q.current) * m];
   if (isnan(mid)) return;
+  // The middle slot may have been dequeued by now (windows of one, three or
+  // five samples, and ones that a run or a finalization left with a few):
+  // its value is then no longer among the live ones, and DENSE's extremum,
+  // one of them, need not equal it.
+  const bool gone = (q.current >= q.start ? q.current - q.start : q.current - q.start + w) >= q.live;
   bool above = false, below = false;
   if (q.same >= q.live && mid == win[static_cast<size_t>(q.end) * m]) {
     // every live value equals the newest one, and so mid (a run of equal
@@ -612,15 +617,10 @@ __device__ __forceinline__ void osc_check(const OscRef& o, const OscQueue& q, co
     left -= 8;
   }
   if (above && below) return;
-  // The middle slot may have been dequeued by now (windows of one, three or
-  // five samples, and ones that a run or a finalization left with a few):
-  // its value is then no longer among the live ones, and DENSE's extremum,
-  // one of them, need not equal it.
-  int ahead = q.current - q.start;
-  if (ahead < 0) ahead += w;
-  if (ahead >= q.live) {
+  if (gone) {
     bool equal = false;
     int at = q.start;
+#pragma unroll 1  // (rare; unrolled it costs the usual path 2 %)
     for (int u = 0; u < q.live; ++u) {
       equal = equal || win[static_cast<size_t>(at) * m] == mid;
       at = (at == w - 1) ? 0 : at + 1;
