@@ -25,6 +25,16 @@ constexpr int kValsPad = 2;        // register kernel: doubles between the rows 
 constexpr int kStepSmem2 = 100000 + 8 * kValsPad * kNS;
 constexpr int kStepSmem1 = 200000 + 8 * kValsPad * kNS;
 constexpr int kIndexSlots = 64;    // queue indices of oscillation analyses that a CTA shares
+// Register kernel: the step's rows of a model's reads and writes, kept as a
+// table in static shared memory, beside a CTA's parameters and the largest
+// dynamic share within the 227 KB a CTA may have; up to 384 (delay reaction,
+// species) pairs, and models too large for it form their rows per read.
+constexpr int kPairs = kND * kNS;
+constexpr int kTableBytes = 16 * (2 * kPairs + kNS) + 12 * (2 * kPairs + kNS);
+constexpr int kStepStatic = 8 * kPairs + 8 * kNP + 12 * kNS + 16 * kIndexSlots + 8 * kMaxAnalyses + 256;
+constexpr int kCtaSmem = 227 * 1024;
+constexpr bool kRowTables =
+    kPairs > 0 && kPairs <= 384 && kStepSmem1 + kStepStatic + kTableBytes <= kCtaSmem;
 constexpr int kMaxCluster = 16;    // register kernel: CTAs a set's cells may be spread over (above the portable 8)
 constexpr int kClusterSmem = 100000;  // dynamic shared memory of such a CTA (two per SM)
 constexpr int64_t kMaxRegisterRing = 1 << 25;  // register kernel: elements of one set's history rings

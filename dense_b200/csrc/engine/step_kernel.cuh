@@ -377,11 +377,6 @@ struct RegContext {
   }
 };
 
-// The tables of RegContext fit in static shared memory up to this many
-// (delay reaction, species) pairs; models above it form their rows per read.
-constexpr int kPairs = kND * kNS;
-constexpr bool kRowTables = kPairs > 0 && kPairs <= 384;  // 64 bytes a pair
-
 // ------------------------------------------------------------ analyses
 // All per-cell analysis state is structure-of-arrays over the analysed
 // cells, so the threads of a warp touch consecutive doubles.
