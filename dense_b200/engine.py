@@ -224,16 +224,17 @@ def _describe(L, sets, analyses, step_size, analysis_interval, precision, device
     keep = []
     cset = (_SetDesc * len(sets))()
     rows = np.frombuffer(cset, _SET_DTYPE)
-    known = {}  # arrays that several sets share, by id (all alive during this call)
+    known = {}  # id -> (address, array): arrays that several sets share; held, since a set may make them on access
 
     def address(a):
         if a is None:
             return 0
         at = known.get(id(a))
         if at is None:
-            at = known[id(a)] = a.__array_interface__["data"][0]
-        return at
+            at = known[id(a)] = a.__array_interface__["data"][0], a
+        return at[0]
 
+    keep.append(known)
     for s in sets:
         if s.cell_params is not None and s.cell_params.size != s.num_cells * L.num_params:
             raise DenseError("cell_params must be [num_cells][num_params]")
@@ -299,8 +300,8 @@ class Batch:
         self.precision = precision
         self.device = device
         L = self.L
-        run, cset, self._keep = _describe(L, self.sets, self.analyses, step_size, analysis_interval, precision,
-                                          device)
+        # (the library copies what it is given: the arrays need to live during the call only)
+        run, cset, keep = _describe(L, self.sets, self.analyses, step_size, analysis_interval, precision, device)
         h = C.c_void_p()
         L._check(L.lib.dense_engine_create(C.byref(run), len(self.sets), cset, C.byref(h)))
         self.h = h
