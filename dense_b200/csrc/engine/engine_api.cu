@@ -345,8 +345,9 @@ int plan_set(const dense_set_desc& in, double dt, int elem_bytes, SetPlan& plan,
   const bool ordered = tr.ordered, bad = tr.bad;
   if (bad) plan.status |= kSetBadDelay;
   // sets whose neighbour reads see the row written in the same step, and
-  // sets larger than a CTA, run in the memory-state kernel, which keeps
-  // every species in its ring (at least two rows)
+  // sets larger than a CTA, keep every species in its ring (at least two
+  // rows), as the memory-state and wave kernels need; of the latter those
+  // that a cluster holds run in the register kernel (ranks, below)
   d.ordered = ordered ? 1 : 0;
   plan.use_mem = ordered || n > kStepThreads || force_mem;
   plan_levels(in, ordered, plan);
@@ -385,8 +386,8 @@ int plan_set(const dense_set_desc& in, double dt, int elem_bytes, SetPlan& plan,
     }
   };
   stage();
-  // the register kernel forms ring offsets in 32 bits and packs lags in 26;
-  // larger rings (no model's delays come near) go to the memory kernel
+  // the register kernel forms ring offsets in 32 bits, flags in the upper
+  // two; larger rings (no model's delays come near) go to the memory kernel
   if (off > kMaxRegisterRing) plan.ranks = 0;
   if (!plan.use_mem && off > kMaxRegisterRing) {
     plan.use_mem = true;

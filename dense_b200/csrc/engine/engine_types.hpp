@@ -17,7 +17,7 @@ constexpr int kNR = NUM_REACTIONS;
 constexpr int kND = NUM_DELAY_REACTIONS;
 constexpr int kNP = NUM_PARAMS;
 constexpr int kMaxAnalyses = 8;
-constexpr int kStepThreads = 256;  // register kernel: one thread per cell, one CTA per set
+constexpr int kStepThreads = 256;  // register kernel: most cells (threads) of a CTA
 constexpr int kMaxCells = 65536;   // memory kernel: cells per set
 constexpr int kValsPad = 2;        // register kernel: doubles between the rows of the sampled state
 // Register kernel: dynamic shared memory of a CTA, of two and of one per SM
@@ -37,7 +37,9 @@ constexpr bool kRowTables =
     kPairs > 0 && kPairs <= 384 && kStepSmem1 + kStepStatic + kTableBytes <= kCtaSmem;
 constexpr int kMaxCluster = 16;    // register kernel: CTAs a set's cells may be spread over (above the portable 8)
 constexpr int kClusterSmem = 100000;  // dynamic shared memory of such a CTA (two per SM)
-constexpr int64_t kMaxRegisterRing = 1 << 25;  // register kernel: elements of one set's history rings
+// Register kernel: elements of one set's history rings.  A resolved read is an
+// offset into them or a lag, with two flags in the bits from 2^30 on.
+constexpr int64_t kMaxRegisterRing = 1 << 25;
 
 // Per-set status bits (also the public DENSE_SET_* values).
 enum : int {

@@ -1,13 +1,16 @@
-// The batched deterministic step kernel for one DENSE model, templated on
+// The batched deterministic step kernels for one DENSE model, templated on
 // the arithmetic type T (double: the exact FP64 engine; float: the FP32
 // engine with Kahan-compensated state updates).
 //
-// Mapping: one CTA per parameter set, one thread per tissue cell.  A launch
+// Mapping of the register kernel: one thread per tissue cell; a parameter set
+// is one CTA, or above 256 cells a cluster of up to 16.  (The memory and wave
+// kernels, below, walk a set with one CTA.)  A launch
 // runs the chunked time loop of DENSE's run_simulation
 // (run_simulation.hpp:127-157) for every set from its current chunk up to
 // StepArgs::chunk_count more chunks: at each chunk boundary the fused analyses sample the
-// state, then (int)(interval/dt) Euler steps follow.  One __syncthreads per
-// step separates the writes of step n from the neighbour reads of step n+1.
+// state, then (int)(interval/dt) Euler steps follow.  One barrier per step,
+// of the CTA or the cluster, separates the writes of step n from the reads
+// of that row in step n+1; reads of older rows are issued ahead of it.
 //
 // State: each thread keeps its cell's lag-0 concentrations in registers.
 // Only species whose history is read (found by tracing the model's
@@ -177,6 +180,7 @@ struct DeviceContext {
 constexpr int kReadLag0 = static_cast<int>(0x80000000u);     // row tables: an own read of lag 0
 constexpr int kReadChecked = static_cast<int>(0xC0000000u);  // a flagged read
 constexpr int kReadCheckBit = 0x40000000;
+static_assert(kMaxRegisterRing <= kReadCheckBit, "row offsets must stay below the flag bits");
 
 // getCon(sp, k): lag (k - 1) mod S.
 __device__ __forceinline__ int resolve_own(int k, int S, int mask) {

@@ -93,7 +93,7 @@ _KERNELS = {}
 
 
 def synchrony_batch(X, counts):
-    """synchrony() of every set at once on the GPU (one CTA per set,
+    """synchrony() of every set at once on the GPU (a cluster of CTAs per set,
     csrc/surrogate/features.cu): X [sets][samples][cells] (a float64 CUDA
     tensor, cells contiguous; rows past a set's count are ignored), counts
     [sets]; float64 numpy array out."""
