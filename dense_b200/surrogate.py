@@ -369,11 +369,13 @@ class MLP:
         on the GPU (a float tensor [B][n_in]); nothing crosses to the host.
         One launch carries every row through the whole network; inputs of
         another type or layout are converted `batch` rows at a time."""
-        out = self.torch.empty((X.shape[0], self.n_out), device=self.dev)
         packed = self._pack()
-        step = max(1, X.shape[0]) if self._as_rows(X) else batch
-        for s in range(0, X.shape[0], step):
-            self.k.predict(self._rows(X[s:s + step]), packed, self.b, out[s:s + step])
+        out = self.torch.empty((X.shape[0], self.n_out), device=self.dev)
+        if self._as_rows(X):
+            self.k.predict(X, packed, self.b, out)
+        else:
+            for s in range(0, X.shape[0], batch):
+                self.k.predict(self._rows(X[s:s + batch]), packed, self.b, out[s:s + batch])
         self.k.check()
         return out
 
