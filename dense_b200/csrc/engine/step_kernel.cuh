@@ -854,7 +854,7 @@ __device__ __forceinline__ bool analyses_sample(const StepArgs& a, double* anl, 
 // cells each), which meet at a cluster barrier after each step; for tissues
 // of more than 256 cells.  The memory kernel, which walks such a set with one
 // CTA and keeps the state in the rings, took 4.82 ms for 96 sets x 733 cells
-// x 200 steps; three CTAs a set take 2.84 ms, and 93 sets, all the clusters
+// x 200 steps; three CTAs a set take 2.65 ms, and 93 sets, all the clusters
 // of three that the GPU holds at once, 1.02 ms (5.1 us a step, of which the
 // cluster barrier and the release of the rows written before it are a
 // quarter).
