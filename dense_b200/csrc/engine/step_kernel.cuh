@@ -1459,7 +1459,8 @@ struct WaveContext {
   }
 
   // (checks set error bits without leaving the straight-line path; a set
-  // with an error bit is reported, not its values)
+  // with an error bit is reported, not its values: a read of a row that is
+  // not kept takes one that is)
   __device__ __forceinline__ T own(specie_id sp, int k) const {
     const int s = ring_size(sp);
     int lag = k - 1;
@@ -1469,8 +1470,9 @@ struct WaveContext {
       lag = ((k - 1) % s + s) % s;
     }
     if (lag == 0) return cur[sp];
-    *err |= lag >= D[sp] ? kSetUnstagedLag : 0;
-    return row(sp, lag)[cell];
+    const bool kept = lag < D[sp];
+    *err |= kept ? 0 : kSetUnstagedLag;
+    return row(sp, kept ? lag : 0)[cell];
   }
 
   __device__ __forceinline__ T own_lag(specie_id sp, int lag) const {
@@ -1514,7 +1516,7 @@ struct WaveContext {
       return average(sum);
     }
     *err |= lag >= D[sp] - 1 ? kSetUnstagedLag : 0;
-    return nbr_lag(sp, lag);
+    return nbr_lag(sp, lag < D[sp] ? lag : 0);
   }
 
   __device__ __forceinline__ T getCon(specie_id sp) const { return cur[sp]; }

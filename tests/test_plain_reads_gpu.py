@@ -77,3 +77,18 @@ def test_late_flagged_reads(cells):
     assert np.array_equal(flags, want_flags)
     for g, w in zip(got, want):
         assert np.array_equal(g, w)
+
+
+def test_late_flagged_reads_in_shared_rows():
+    """The wave kernel keeps exactly the rows that the planning asked for; a
+    read further back is flagged and stays within them."""
+    from dense_b200 import engine as E
+    lib = X.engine_library(*MODEL)
+    for cells in (1, 40, 200):
+        sets = _sets(cells, False, (30.0, 4.0, 6.0, 3.0), 7, schedule=E.SCHEDULE_SHARED_ROWS)
+        states, flags = X.engine_states(lib, sets, 0.01, 0.1)
+        assert (flags == 4).any() and all(np.isfinite(x).all() for x in states)
+        sets = _sets(cells, False, (7.0, 4.0, 6.0, 3.0), 7, schedule=E.SCHEDULE_SHARED_ROWS)
+        want = X.oracle_states(X.oracle_library(*MODEL), sets, 0.01, 0.1)
+        states, flags = X.engine_states(lib, sets, 0.01, 0.1)
+        assert (flags == 0).all() and all(np.array_equal(x, y) for x, y in zip(states, want))
