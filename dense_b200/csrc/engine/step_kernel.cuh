@@ -1423,6 +1423,11 @@ __global__ void __launch_bounds__(256, 2) dense_step_mem_kernel(const StepArgs a
 // memory; a cell's neighbour ids come from its 16-byte record.
 template <typename T, bool kUniform>
 struct WaveContext {
+  // Whether each species' row of lag S-1 is kept beside its other rows: with
+  // two species they save their forming at every read; with 14 they are 28
+  // more registers of 128 (300 unordered sets of 200 cells x 50 steps with
+  // shared rows 0.750 ms with them, 0.745 without).
+  static constexpr bool kCacheLast = kNS <= 8;
   const T* cur;            // this cell's lag-0 state [NS] (registers)
   const T* prm;            // parameters: shared row (pstride 1) or this cell's column (pstride n)
   int pstride;
@@ -1431,7 +1436,7 @@ struct WaveContext {
   const int* r0;           // row holding lag 0, per species (registers)
   T* const* base;          // row 0 of each species, shared or global (registers)
   T* const* wrow;          // the row this step writes, per species (registers)
-  T* const* last;          // the row of lag S-1, per species (registers)
+  T* const* last;          // kCacheLast: the row of lag S-1, per species (registers)
   const uint16_t* nbr;     // this cell's neighbour ids, ascending (registers; 0 past the count)
   int nnbr;
   int lower;               // of them, below this cell's id (the first ones)
@@ -1505,7 +1510,7 @@ struct WaveContext {
     if (lag == s - 1 && s > 1) {
       *err |= D[sp] < s + 1 ? kSetOrderedReads : 0;
       const T* fresh = wrow[sp];
-      const T* old = last[sp];
+      const T* old = kCacheLast ? last[sp] : row(sp, lag < D[sp] ? lag : 0);
       T v[kWaveMaxNbrs];
 #pragma unroll
       for (int e = 0; e < kWaveMaxNbrs; ++e) v[e] = (e < lower ? fresh : old)[nbr[e]];
@@ -1577,7 +1582,11 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_wave_kernel(c
   const SetProgress pg = a.prog[set];
   if ((pg.status & (kSetDropped | kSetNotRunnable)) || pg.finalized) return;
 
-  const int pstride = kUniform ? 0 : sd.param_stride;
+  // Known to be 0, it lets the compiler hold the set's parameters in registers
+  // over the steps.  The grid's six fit, and 47 in FP32 (0.54 -> 0.50 ms); 47
+  // in FP64 were spilled instead (300 unordered sets of 200 cells x 50 steps
+  // with shared rows: 1.16 ms, and 0.75 with the stride read).
+  const int pstride = kUniform && kNP * sizeof(T) <= 192 ? 0 : sd.param_stride;
   const T* P = static_cast<const T*>(a.params) + sd.param_base;
   T* ring = static_cast<T*>(a.ring) + sd.ring_base;
   for (int i = tid; i <= kWaveMaxNbrs; i += blk) s_rc[i] = i > 0 ? T(1) / static_cast<T>(i) : T(0);
@@ -1655,14 +1664,16 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_wave_kernel(c
   T* lbase[kNS];
   T* lcur[kNS];
   T* lw[kNS];
-  T* llast[kNS];
+  constexpr bool kCacheLast = WaveContext<T, kUniform>::kCacheLast;
+  T* llast[kCacheLast ? kNS : 1];
 #pragma unroll
   for (int sp = 0; sp < kNS; ++sp) {
     lS[sp] = kND == 0 ? 2 : s_S[sp];
     lD[sp] = s_D[sp];
     lbase[sp] = kAllShared ? reinterpret_cast<T*>(w_dyn + sd.smem_off[sp]) : s_base[sp];
     r0[sp] = 0;
-    lcur[sp] = lw[sp] = llast[sp] = lbase[sp];
+    lcur[sp] = lw[sp] = lbase[sp];
+    if constexpr (kCacheLast) llast[sp] = lbase[sp];
   }
   // thread groups, one per wavefront
   const int fronts = sd.wave_fronts;
@@ -1729,13 +1740,20 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) dense_step_wave_kernel(c
           fresh_step = false;
 #pragma unroll
           for (int sp = 0; sp < kNS; ++sp) {
-            r0[sp] = static_cast<int>((step + kk) % lD[sp]);
+            if (kk == grp) {
+              r0[sp] = static_cast<int>((step + kk) % lD[sp]);
+            } else {  // this group's step before was `fronts` rows back
+              r0[sp] += fronts;
+              while (r0[sp] >= lD[sp]) r0[sp] -= lD[sp];
+            }
             const int rw = r0[sp] + 1 == lD[sp] ? 0 : r0[sp] + 1;
-            // (a row of lag S-1 exists where a set reads it)
-            const int rl = r0[sp] - (lS[sp] - 1 < lD[sp] ? lS[sp] - 1 : 0);
             lcur[sp] = lbase[sp] + r0[sp] * n;
             lw[sp] = lbase[sp] + rw * n;
-            llast[sp] = lbase[sp] + (rl < 0 ? rl + lD[sp] : rl) * n;
+            if constexpr (kCacheLast) {
+              // (a row of lag S-1 exists where a set reads it)
+              const int rl = r0[sp] - (lS[sp] - 1 < lD[sp] ? lS[sp] - 1 : 0);
+              llast[sp] = lbase[sp] + (rl < 0 ? rl + lD[sp] : rl) * n;
+            }
           }
         }
         const int i1 = t_lvl[l + 1];
