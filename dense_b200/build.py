@@ -17,7 +17,7 @@ import concurrent.futures as cf
 import os
 import subprocess
 
-from .models import MODEL_DIRS, model_dir
+from .models import MODEL_DIRS, MissingModelError, model_dir
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -71,7 +71,7 @@ def build_model(model, force=False, verbose=False):
     if mdir is None or not os.path.isdir(mdir):
         if os.path.exists(out):
             return out
-        raise RuntimeError("DENSE model directory %s not found and no prebuilt %s" % (mdir, out))
+        raise MissingModelError("DENSE model directory %s not found and no prebuilt %s" % (mdir, out))
     deps = _sources() + [os.path.join(mdir, f) for f in os.listdir(mdir)]
     if not force and _up_to_date(out, deps):
         return out

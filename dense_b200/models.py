@@ -25,6 +25,11 @@ MODEL_DIRS = {
 ENV = "DENSE_REF_DIR"
 
 
+class MissingModelError(RuntimeError):
+    """A model whose headers are not on this machine and that was not built
+    before."""
+
+
 def dense_dir(required=True):
     """The DENSE source tree named by $DENSE_REF_DIR.
 
@@ -37,8 +42,8 @@ def dense_dir(required=True):
     if not required:
         return None
     why = "is not set" if not d else "names %r, which is not a directory" % d
-    raise RuntimeError("%s %s: set it to a DENSE source tree (the directory holding models/ and source/)"
-                       % (ENV, why))
+    raise MissingModelError("%s %s: set it to a DENSE source tree (the directory holding models/ and source/)"
+                            % (ENV, why))
 
 
 def model_dir(key, required=True):

@@ -34,7 +34,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 sys.path.insert(0, ROOT)
 
-from dense_b200.models import MODEL_DIRS, dense_dir, model_dir  # noqa: E402
+from dense_b200.models import MODEL_DIRS, MissingModelError, dense_dir, model_dir  # noqa: E402
 
 LIB_DIR = os.path.join(HERE, "_lib")
 REF_DIR = os.path.join(HERE, "_ref")
@@ -116,7 +116,7 @@ def build_oracle(model, force=False):
     if mdir is None or not os.path.isdir(mdir):
         if os.path.exists(out):
             return out
-        raise RuntimeError("model directory %s not found and no prebuilt %s" % (mdir, out))
+        raise MissingModelError("model directory %s not found and no prebuilt %s" % (mdir, out))
     if not force and _newer(out, [src, hdr]):
         return out
     os.makedirs(LIB_DIR, exist_ok=True)

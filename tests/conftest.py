@@ -30,3 +30,27 @@ def pytest_collection_modifyitems(config, items):
     for item in items:
         if "gpu" in item.keywords:
             item.add_marker(skip)
+
+
+def _skip_without_tree(outcome):
+    """Tests of DENSE's own models need its headers, or libraries built from
+    them before.  On a machine with neither they are skipped, and those of
+    the models written out in tests/ run; with a DENSE tree a model that is
+    missing fails its test."""
+    from dense_b200.models import ENV, MissingModelError
+    tree = os.environ.get(ENV)
+    error = outcome.exception
+    # (a rank of its own process reports the error in its traceback)
+    missing = isinstance(error, MissingModelError) or "models.MissingModelError: " in str(error)
+    if error is not None and missing and not (tree and os.path.isdir(os.path.join(tree, "models"))):
+        outcome.force_exception(pytest.skip.Exception(str(error)))
+
+
+@pytest.hookimpl(hookwrapper=True)
+def pytest_runtest_setup(item):
+    _skip_without_tree((yield))
+
+
+@pytest.hookimpl(hookwrapper=True)
+def pytest_runtest_call(item):
+    _skip_without_tree((yield))
