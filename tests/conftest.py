@@ -41,8 +41,9 @@ def _skip_without_tree(outcome):
     tree = os.environ.get(ENV)
     error = outcome.exception
     # (a rank of its own process reports the error in its traceback)
-    missing = isinstance(error, MissingModelError) or "models.MissingModelError: " in str(error)
-    if error is not None and missing and not (tree and os.path.isdir(os.path.join(tree, "models"))):
+    rank = type(error).__name__ == "ProcessRaisedException"
+    missing = isinstance(error, MissingModelError) or (rank and "models.MissingModelError: " in str(error))
+    if missing and not (tree and os.path.isdir(os.path.join(tree, "models"))):
         outcome.force_exception(pytest.skip.Exception(str(error)))
 
 

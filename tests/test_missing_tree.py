@@ -2,6 +2,7 @@
 failed where the tree is there."""
 
 import pytest
+from torch.multiprocessing import ProcessRaisedException
 
 from dense_b200.models import ENV, MissingModelError, model_dir
 from tests import conftest
@@ -17,9 +18,10 @@ class _Outcome:
 
 @pytest.mark.parametrize("error,skips", [
     (MissingModelError("model directory x not found"), True),
-    (RuntimeError("in a rank: dense_b200.models.MissingModelError: x"), True),
+    (ProcessRaisedException("dense_b200.models.MissingModelError: x", 1, 2), True),
+    (ProcessRaisedException("AssertionError", 1, 2), False),
     (RuntimeError("nvcc failed"), False),
-    (AssertionError("state differs"), False),
+    (AssertionError("a program's output: dense_b200.models.MissingModelError: x"), False),
     (None, False)])
 @pytest.mark.parametrize("tree", [None, "empty", "dense"])
 def test_missing_models(error, skips, tree, tmp_path, monkeypatch):
