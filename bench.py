@@ -530,6 +530,14 @@ def run_reference(a):
     if rank != 0:
         return
     import multiprocessing as mp
+    from dense_b200.models import MissingModelError
+    from oracle.pyoracle import load_oracle, load_ref
+    try:
+        if load_ref("her_model_2014") is None:
+            load_oracle("her_model_2014")
+    except MissingModelError as e:
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+        return
     cores = len(os.sched_getaffinity(0))
     ctx = mp.get_context("spawn")
     minutes = 60.0
